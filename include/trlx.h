@@ -382,7 +382,9 @@ typedef struct {
 } trlx_stats;
 
 #define TRLX_K_SPMV 0      /* built-in operator (+ fused alpha)          */
-#define TRLX_K_PROJECT 1   /* Gram-Schmidt projection h = V^H r          */
+#define TRLX_K_PROJECT 1   /* Gram-Schmidt projection h = V^H r (with the
+                              update of the vector before it where a step is
+                              a single sweep over the basis)               */
 #define TRLX_K_UPDATE 2    /* Gram-Schmidt update r - V h                */
 #define TRLX_K_NORMALIZE 3 /* scaling / storing the new basis vector     */
 #define TRLX_K_RITZ 4      /* restart recombination V Y                  */

@@ -174,6 +174,17 @@ __device__ __forceinline__ void store_c(zd *p, const zd (&o)[R]) {
     for (int k = 0; k < R; ++k) *reinterpret_cast<double2 *>(p + k) = make_double2(o[k].x, o[k].y);
 }
 
+// ---- asynchronous copies into shared memory (16 bytes per thread) -------------
+__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
 // ---- deterministic reductions ------------------------------------------------
 // Sum over the block in a fixed tree order; result valid in thread 0.
 template <class C>

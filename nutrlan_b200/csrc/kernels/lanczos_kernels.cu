@@ -282,16 +282,6 @@ constexpr size_t async_smem() {
     return (size_t)NW * NS * CPW * 32 * 16;
 }
 
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
 template <class T, int NW, int CPW, int NS>
 __global__ void __launch_bounds__(NW * 32, 1)
     k_project_async(T *const *__restrict__ cols, int m, long n_pad, long chunk,
