@@ -305,8 +305,14 @@ struct RowCfg {
     static constexpr int kAcc = 2 * kLanes;  // TMEM accumulators of 32 columns
     static_assert(kAcc % kEpi == 0, "an accumulator belongs to one epilogue warpgroup");
     static constexpr int kThreads = 32 * (4 * kEpi + 1 + kLanes);
-    static constexpr int kCols = kAcc * kCh;
-    static_assert(kCols >= 32 && kCols <= 512 && (kCols & (kCols - 1)) == 0, "TMEM allocations are powers of two");
+    // Lane m waits for full[s] by phase parity alone, so it must have seen
+    // every earlier phase of its stages: a stage belongs to one lane.  (With
+    // six stages for four lanes a lane could pass on the phase before its
+    // own, whose loads another lane had still to wait for.)
+    static_assert(kStages % kLanes == 0, "a stage belongs to one MMA lane");
+    static constexpr int pow2(int c) { return c <= 32 ? 32 : (c <= 64 ? 64 : (c <= 128 ? 128 : (c <= 256 ? 256 : 512))); }
+    static constexpr int kCols = pow2(kAcc * kCh);  // TMEM allocations are powers of two
+    static_assert(kAcc * kCh <= 512, "TMEM columns");
     static constexpr int kOffA = kWBytes;
     static constexpr int kOffO = kOffA + kStages * 3 * kRowBuf;  // 4*kEpi warps x 2 buffers of 2 KB
     static constexpr int kOffBar = kOffO + 4 * kEpi * 2 * 2048;
@@ -461,13 +467,12 @@ __global__ void __launch_bounds__(RowCfg<kLanes, kEpi, kStages>::kThreads, 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Cfg::kCols) : "memory");
 }
 
-// The configuration the library launches: four MMA lanes, two epilogue
-// warpgroups, six stages (213 KB of shared memory, 416 threads).  Measured
-// per 32 -> 32 layer at 256 x 256, batch 16: 1 lane 66 us, 2 lanes 41 us,
-// 4 lanes with one epilogue warpgroup 41 us (the epilogue bound), 4 lanes
-// with two 37 us; every configuration bitwise equal to the 9-tap kernel.
-using RowsCfg = RowCfg<4, 2, 6>;
-constexpr auto *kRowsKernel = &k_conv_rows<4, 2, 6>;
+// The configuration the library launches: three MMA lanes, two epilogue
+// warpgroups, six stages (213 KB of shared memory, 384 threads): 0.58 ms a
+// forward pass at 256 x 256, batch 32 (0.21 ms at batch 8); every
+// configuration is bitwise equal to the 9-tap kernel.
+using RowsCfg = RowCfg<3, 2, 6>;
+constexpr auto *kRowsKernel = &k_conv_rows<3, 2, 6>;
 
 // ---------------------------------------------------------------------------
 // Weight gradient on tcgen05: dW[tap][ci][co] = sum_p in[p + off(tap)][ci] *
