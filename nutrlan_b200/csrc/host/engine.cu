@@ -184,8 +184,8 @@ Options options_from(const trlx_options *o) {
 
 namespace {
 
-// Vectors shorter than this take their steps with the discrete kernels (or,
-// in CSR form, the cooperative one).
+// FP64 and complex128 vectors shorter than this take their steps in the
+// cooperative kernel instead of sweeps.
 constexpr long kSweepMinRows = 1L << 17;
 
 enum Scal { kAlpha = 0, kR2Pre = 1, kH2 = 2, kR2Post = 3, kNorm = 4, kNumScal = 8 };
@@ -280,7 +280,14 @@ class Engine {
     int refine_fp64(int k, double *max_res);
     bool spec_enabled() const;
     int spec_segment(int *jnd, int S, int kept);
+    // Asked of every beta of a run of single-sweep steps: keeps |r|^2 and
+    // r^H A r, formed from unnormalised vectors, far from overflow and
+    // underflow.  A solve that meets another goes on without such runs.
+    bool scale_off_ = false;
+    static bool in_range(double beta) { return beta > 1e-90 && beta < 1e90; }
     bool sweeps(int jnd) const;
+    bool coop_steps(int jnd) const;
+    int upload_run(int j0, int kept);
     int sweep_steps(int j0, int S, int kept);
     bool accept_step(int jnd, int kept, const double *lg, bool sweep);
     void track_ritz(int nd) {
@@ -518,10 +525,10 @@ int Engine<T>::setup() {
     }
     // Small buffers carved from one allocation (256-byte aligned pieces).
     auto al = [](size_t b) { return (b + 255) / 256 * 256; };
-    const size_t b_coef = al(sizeof(double) * sweep_doubles()), b_scal = al(sizeof(double) * kNumScal),
-                 b_Y = al(sizeof(double) * (size_t)maxlan_ * maxlan_), b_cols = al(sizeof(T *) * P_),
-                 log_len = 4 * ((size_t)maxlan_ + 2), b_log = al(sizeof(double) * log_len);
-    if (!Workspace::ensure(&ws.small, &ws.small_bytes, b_coef + b_scal + b_Y + b_cols + b_log)) return -5;
+    const size_t log_len = 4 * ((size_t)maxlan_ + 2), b_coef = al(sizeof(double) * (sweep_doubles() + log_len)),
+                 b_scal = al(sizeof(double) * kNumScal), b_Y = al(sizeof(double) * (size_t)maxlan_ * maxlan_),
+                 b_cols = al(sizeof(T *) * P_);
+    if (!Workspace::ensure(&ws.small, &ws.small_bytes, b_coef + b_scal + b_Y + b_cols)) return -5;
     char *sp = static_cast<char *>(ws.small);
     d_coef_ = reinterpret_cast<C *>(sp);
     d_sc_c_ = d_coef_ + P_;
@@ -529,11 +536,11 @@ int Engine<T>::setup() {
     d_sc_tb_ = d_sc_ta_ + P_;
     d_sc_s_ = d_sc_tb_ + P_;
     d_sc_dot_ = d_sc_s_ + 4;
+    d_log_ = d_sc_s_ + 8;  // read back together with the flag before it
     d_scal_ = reinterpret_cast<double *>(sp + b_coef);
     d_Y_ = reinterpret_cast<double *>(sp + b_coef + b_scal);
     d_cols_ = reinterpret_cast<T **>(sp + b_coef + b_scal + b_Y);
-    d_log_ = reinterpret_cast<double *>(sp + b_coef + b_scal + b_Y + b_cols);
-    const size_t host_len = log_len + sweep_doubles();
+    const size_t host_len = 4 + log_len + sweep_doubles();
     if (ws.h_log_len < host_len) {
         cudaFreeHost(ws.h_log);
         ws.h_log = nullptr;
@@ -541,7 +548,7 @@ int Engine<T>::setup() {
         CK(cudaMallocHost(&ws.h_log, sizeof(double) * host_len));
         ws.h_log_len = host_len;
     }
-    h_log_ = ws.h_log;
+    h_log_ = ws.h_log + 4;
     h_sweep_ = h_log_ + log_len;
     CK(cudaMemsetAsync(d_scal_, 0, sizeof(double) * kNumScal, st_));
     if (!ws.h_scal) CK(cudaMallocHost(&ws.h_scal, sizeof(double) * kNumScal));
@@ -1116,15 +1123,21 @@ bool Engine<T>::spec_enabled() const {
 }
 
 // Whether the speculative steps from basis size jnd on run as single sweeps
-// (sweep.h).  The range of the last beta keeps |r|^2 and r^H A r, formed
-// from unnormalised vectors, far from overflow and underflow.
+// (sweep.h).
 template <class T>
 bool Engine<T>::sweeps(int jnd) const {
-    if (n_pad_ < kSweepMinRows || jnd + 1 > kSweepCols) return false;
+    // A 32-bit basis has no other speculative steps, so any length counts.
+    if ((kWide && n_pad_ < kSweepMinRows) || jnd < 1 || jnd + 1 > kSweepCols || scale_off_) return false;
     if ((size_t)P_ * n_pad_ * sizeof(T) > (1ull << 36)) return false;  // 32-bit column offsets, 16-byte units
-    const double b = beta_[jnd - 1];
-    if (!(b > 1e-90 && b < 1e90)) return false;
     const char *e = std::getenv("TRLX_SWEEP");
+    return !(e && e[0] == '0');
+}
+
+// Whether they run in the cooperative kernel (coop.h).
+template <class T>
+bool Engine<T>::coop_steps(int jnd) const {
+    if (!kWide || jnd < 1 || n_pad_ >= kSweepMinRows || scale_off_) return false;
+    const char *e = std::getenv("TRLX_COOP");
     return !(e && e[0] == '0');
 }
 
@@ -1160,17 +1173,46 @@ bool Engine<T>::accept_step(int jnd, int kept, const double *lg, bool sweep) {
     const double rnrm = std::sqrt(r2post);
     if (!(rnrm > DBL_MIN)) return false;
     if (rnrm <= DBL_EPSILON * std::fabs(alpha) || jnd >= info_->ntot) return false;
-    if (sweep && !(rnrm > 1e-90 && rnrm < 1e90)) return false;  // as in sweeps()
+    if (sweep && !in_range(rnrm)) {
+        scale_off_ = true;
+        return false;
+    }
     alpha_[jnd - 1] = alpha;
     beta_[jnd - 1] = rnrm;
     alfrot_[jnd - 1] = alpha;
     betrot_[jnd - 1] = rnrm;
-    fl_ += 6 * nrow_;
+    fl_ += jm1 == kept ? 2.0 * jnd * nrow_ + 2.0 * nrow_ : 6.0 * nrow_;
     const double f1 = fl_;
     fl_ += fo + 4.0 * nrow_ * jnd + nrow_;
     fl_h_ += fl_ - f1;
     info_->north++;
     return true;
+}
+
+// What a run of single-sweep steps from basis size j0 starts from: T, and
+// the first product's coefficients (it is of a finished vector: nothing to
+// correct, scale 1).
+template <class T>
+int Engine<T>::upload_run(int j0, int kept) {
+    std::memset(h_sweep_, 0, sizeof(double) * sweep_doubles());
+    double *hc = h_sweep_ + (sizeof(C) / sizeof(double)) * (size_t)P_;
+    double *hta = hc + (sizeof(C) / sizeof(double)) * (size_t)P_, *htb = hta + P_, *hs = htb + P_;
+    // The step after a restart (j0 == kept) has the arrowhead row for its
+    // recurrence, the others the column before (32-bit storage: from its
+    // FP64 copy, with the scalar below).
+    const size_t cw = sizeof(C) / sizeof(double);
+    if (j0 == kept)
+        for (int i = 0; i < j0; ++i) hc[cw * i] = beta_[i];
+    else if (kWide)
+        hc[cw * (size_t)(j0 - 1)] = beta_[j0 - 1];
+    for (int i = 0; i < j0; ++i) {
+        hta[i] = alpha_[i];
+        htb[i] = beta_[i];
+    }
+    hs[0] = hs[1] = 1.0;
+    hs[2] = j0 == kept ? 0.0 : beta_[j0 - 1];
+    CK(cudaMemcpyAsync(d_coef_, h_sweep_, sizeof(double) * sweep_doubles(), cudaMemcpyHostToDevice, st_));
+    return 0;
 }
 
 // Issues S single-sweep steps from basis size j0 (sweep.h): per step one
@@ -1179,18 +1221,7 @@ bool Engine<T>::accept_step(int jnd, int kept, const double *lg, bool sweep) {
 // normalisation.  The steps log what the discrete kernels log.
 template <class T>
 int Engine<T>::sweep_steps(int j0, int S, int kept) {
-    std::memset(h_sweep_, 0, sizeof(double) * sweep_doubles());
-    double *hc = h_sweep_ + (sizeof(C) / sizeof(double)) * (size_t)P_;
-    double *hta = hc + (sizeof(C) / sizeof(double)) * (size_t)P_, *htb = hta + P_, *hs = htb + P_;
-    // The first product is of a finished vector: no correction, scale 1.
-    if (kWide) hc[(sizeof(C) / sizeof(double)) * (size_t)(j0 - 1)] = beta_[j0 - 1];
-    for (int i = 0; i < j0; ++i) {
-        hta[i] = alpha_[i];
-        htb[i] = beta_[i];
-    }
-    hs[0] = hs[1] = 1.0;
-    hs[2] = beta_[j0 - 1];
-    CK(cudaMemcpyAsync(d_coef_, h_sweep_, sizeof(double) * sweep_doubles(), cudaMemcpyHostToDevice, st_));
+    if (int e = upload_run(j0, kept)) return e;
     for (int s = 1; s <= S; ++s) {
         const int k = j0 + s - 1;
         SweepArgs<T> w;
@@ -1247,27 +1278,26 @@ template <class T>
 int Engine<T>::spec_segment(int *jnd_io, int S, int kept) {
     const int j0 = *jnd_io;
     cudaEventRecord(ev_[6], st_);
-    bool done = false, sweep = false;
-    // Short CSR problems: the whole run in one cooperative kernel.
+    bool done = false, sweep = false, coop = false;
+    // Short vectors: the whole run in one cooperative kernel.
     if constexpr (kWide) {
-        if (!trlb::op_sell(builtin_) && n_pad_ <= (1L << 18)) {
-            const char *e = std::getenv("TRLX_COOP");
-            if (!(e && e[0] == '0')) {
-                const long part_elems = (long)scratch_.max_blocks * (P_ + 2) * (long)(sizeof(zd) / sizeof(C));
-                int pid = pbeg();
-                const int rc = launch_spec_coop<C>(builtin_, reinterpret_cast<C *const *>(d_cols_), n_pad_,
-                                                   maxlan_ + 1, j0, S, beta_[j0 - 1], d_log_,
-                                                   reinterpret_cast<C *>(scratch_.partials), part_elems, d_coef_, st_);
-                if (rc == -1001) return -1001;
-                if (rc == 0) {
-                    double bytes = 0.0;
-                    for (int s = 1; s <= S; ++s) bytes += spmv_bytes(builtin_) + (2.0 * (j0 + s) + 4.0) * nrow_ * cs();
-                    pend(pid, TRLX_K_OTHER, bytes);
-                    info_->matvec += S;
-                    count_launch();
-                    coop_segments_++;
-                    done = true;
-                }
+        if (coop_steps(j0)) {
+            if (upload_run(j0, kept)) return -1001;
+            int pid = pbeg();
+            const int rc = launch_coop<C>(builtin_, reinterpret_cast<C *const *>(d_cols_),
+                                          reinterpret_cast<C *>(col(maxlan_ + 1)),
+                                          reinterpret_cast<C *>(col(maxlan_ + 2)), n_pad_, j0, S, kept, d_sc_ta_,
+                                          d_sc_tb_, d_log_, d_sc_dot_, static_cast<double *>(scratch_.partials),
+                                          (size_t)scratch_.max_blocks * (P_ + 2) * 2, scratch_.tickets + 5, st_);
+            if (rc == -1001) return -1001;
+            if (rc == 0) {
+                double bytes = 0.0;
+                for (int s = 1; s <= S; ++s) bytes += spmv_bytes(builtin_) + ((double)(j0 + s) + 4.0) * nrow_ * cs();
+                pend(pid, TRLX_K_OTHER, bytes);
+                info_->matvec += S;
+                count_launch();
+                coop_segments_++;
+                done = coop = true;
             }
         }
     }
@@ -1322,7 +1352,8 @@ int Engine<T>::spec_segment(int *jnd_io, int S, int kept) {
         return 0;
     }
     cudaEventRecord(ev_[7], st_);
-    CK(cudaMemcpyAsync(h_log_ + 4, d_log_ + 4, sizeof(double) * 4 * S, cudaMemcpyDeviceToHost, st_));
+    // With the four doubles before the log: the cooperative kernel's flag.
+    CK(cudaMemcpyAsync(h_log_ - 4, d_log_ - 4, sizeof(double) * (4 * S + 8), cudaMemcpyDeviceToHost, st_));
     CK(cudaStreamSynchronize(st_));
     ++syncs_;
     if (!prof_.empty()) flush_prof();
@@ -1330,7 +1361,8 @@ int Engine<T>::spec_segment(int *jnd_io, int S, int kept) {
     cudaEventElapsedTime(&ms, ev_[6], ev_[7]);
     t_orth_ += ms * 1e-3;
     int acc = 0;
-    while (acc < S && accept_step(j0 + acc + 1, kept, h_log_ + 4 * (acc + 1), sweep)) ++acc;
+    if (!(coop && h_log_[-4] != 0.0))
+        while (acc < S && accept_step(j0 + acc + 1, kept, h_log_ + 4 * (acc + 1), sweep || coop)) ++acc;
     const int dropped = S - acc;
     spec_accepted_ += acc;
     info_->matvec -= dropped;
@@ -1607,6 +1639,17 @@ void Engine<T>::run() {
     int j1 = kept;  // columns that map to the caller's evec on exit
 
     while (info->matvec < info->maxmv && info->nec < info->ned) {
+        // ---- steps from the (re)start on, the arrowhead one first -------------
+        int acc = 0;
+        long run = 0;
+        if (spec_enabled() && (sweeps(jnd) || coop_steps(jnd))) {
+            // Up to the next convergence test, which never comes right after
+            // the first step.
+            run = std::min<long>((long)info->klan - jnd, std::max<long>(2, (long)next_test - info->matvec));
+            if (sweeps(jnd)) run = std::min<long>(run, kSweepCols + 1 - jnd);
+            if (run >= 2) acc = std::max(spec_segment(&jnd, (int)run, kept), 0);
+        }
+        if (acc == 0) {
         // ---- first step after (re)start: arrowhead coupling -------------------
         jnd++;
         if (jnd + 1 > maxlan_ + 1 || jnd + 1 >= P_) {
@@ -1656,15 +1699,17 @@ void Engine<T>::run() {
         tm_end();
         if (stat) break;
         rotate_fp64();
-        // Arrow -> tridiagonal for the non-locked part.
+        }
+        // Arrow -> tridiagonal for the non-locked part (the columns up to and
+        // with the first step's).
         for (int i = 0; i < locked; ++i) {
             alfrot_[i] = alpha_[i];
             betrot_[i] = 0.0;
         }
-        i1 = jnd - locked;
+        i1 = kept + 1 - locked;
         arrow_to_tridiag(i1, &alpha_[locked], &beta_[locked], rot_.data(), &alfrot_[locked], &betrot_[locked]);
         fl_ += 8 * i1 * i1 * i1 / 3;
-        betrot_[jnd - 1] = beta_[jnd - 1];
+        betrot_[kept] = beta_[kept];
 
         // ---- regular Lanczos steps ---------------------------------------------
         auto test_convergence = [&]() -> int {
@@ -1683,15 +1728,15 @@ void Engine<T>::run() {
             log_progress();
             return 0;
         };
+        if (acc > 1 && acc == run && info->matvec >= next_test && (stat = test_convergence())) break;
         while (jnd < info->klan && info->nec < info->ned) {
-            if (spec_enabled() && (kWide ? jnd >= 2 || sweeps(jnd) : sweeps(jnd))) {
+            if (spec_enabled() && (kWide ? jnd >= 2 || sweeps(jnd) || coop_steps(jnd) : sweeps(jnd))) {
                 // Steps up to the next convergence test (or the restart).
                 long S = (long)info->klan - jnd;
                 if (sweeps(jnd)) S = std::min<long>(S, kSweepCols + 1 - jnd);
                 if (next_test > info->matvec) S = std::min<long>(S, (long)next_test - info->matvec);
                 else S = 1;
-                S = std::min<long>(S, (long)info->maxmv - info->matvec);
-                if (S >= 2) {
+                if (S >= 2 || (S == 1 && coop_steps(jnd))) {
                     const int acc = spec_segment(&jnd, (int)S, kept);
                     if (acc == S) {
                         if (info->matvec >= next_test && (stat = test_convergence())) break;

@@ -1,5 +1,4 @@
-// Cooperative kernel for runs of speculative Lanczos steps on short vectors
-// (coop.cu).
+// Cooperative kernel for runs of Lanczos steps on short vectors (coop.cu).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -14,24 +13,32 @@ template <class C>
 struct CoopArgs {
     int nrow;
     long n_pad;
-    long chunk;    // rows per block (multiple of 64)
-    int maxcols;   // capacity of h (basis columns)
-    const long long *rp;
+    int chunk;       // rows per block (multiple of 32)
+    int kmax;        // columns the shared arrays hold
+    int nres;        // basis columns kept in shared memory
+    int ecap;        // operator entries kept in shared memory per block (0: none)
+    const long long *ptr;  // CSR row pointers, or SELL-C-32 slice pointers
+    int sell;
+    int tpr;         // lanes per row of the product (a power of two)
     const int *ci;
     const C *va;
     C *const *cols;  // basis column table
+    C *z[2];         // exchange vectors (n_pad rows each)
     int j0, S;       // steps j0 + 1 .. j0 + S
-    double beta0;    // beta of the first step's recurrence
+    int kept;        // leading columns coupled only to column `kept`
+    const double *ta, *tb;  // alphas and betas of the first j0 columns
     double *log;     // [s][4]: alpha, |r|^2 before, |h|^2, |r|^2 after (s = 1..S)
-    C *part;         // (maxcols + 2) * G partials
-    C *h;            // maxcols coefficients
+    double *failed;  // set to 1 when a barrier gave up
+    double *part;    // two sets of the clusters' partial sums
+    unsigned *sync;  // two counters, zero between launches
 };
 
-// Runs S steps (CSR operators only).  Returns 0, -1 if the cooperative
-// kernel does not apply (operator format, device, sizes), -1001 on a CUDA
-// error.
+// Runs S steps of a built-in CSR operator or an unsorted SELL one.  Returns
+// 0, -1 if the kernel does not apply (operator form, device, sizes), -1001
+// on a CUDA error.
 template <class C>
-int launch_spec_coop(const trlx_operator *A, C *const *cols, long n_pad, int maxcols, int j0, int S, double beta0,
-                     double *log, C *part, long part_elems, C *h, cudaStream_t st);
+int launch_coop(const trlx_operator *A, C *const *cols, C *z0, C *z1, long n_pad, int j0, int S, int kept,
+                const double *ta, const double *tb, double *log, double *failed, double *part, size_t part_doubles,
+                unsigned *sync, cudaStream_t st);
 
 }  // namespace trlb
