@@ -6,8 +6,8 @@
 // solve on it: the control flow of the reference's trlanczos
 // (SRC/trlcore.c:723-1532; same usecgs decision, classical Gram-Schmidt pass
 // loop, convergence tests and restart bookkeeping as the host engine), with
-// the projected-problem work done by thread 0 using the very same
-// __host__ __device__ routines as the host engine (dense_core.h,
+// the projected problem on the group's first warp (dense_warp.cuh; the
+// restart decisions by its first lane with the host engine's routines of
 // restart_core.h).  Vector work is block-wide: the operator (5-point
 // stencil with a diagonal, or CSR), alpha and norm reductions, Gram-Schmidt
 // projection/update against the problem's basis, and the restart
@@ -604,14 +604,17 @@ __device__ void solve(const Params &P, int pid, const Grp &G, double *dyn, long 
                 S.alpha[jnd - 1] = a;
             }
             stat = orth<CW>(P, pid, V, ld, n, jnd, true, S.beta[jnd - 2], a, kept, G);
-            if (G.tid == 0) {
-                S.alfrot[jnd - 1] = S.alpha[jnd - 1];
-                S.betrot[jnd - 1] = S.beta[jnd - 1];
+            if (G.tid < 32) {
+                const int lane = G.tid;
+                if (lane == 0) {
+                    S.alfrot[jnd - 1] = S.alpha[jnd - 1];
+                    S.betrot[jnd - 1] = S.beta[jnd - 1];
+                }
+                __syncwarp();
+                int flag = 0;
                 if (!stat && info->matvec >= next_test) {
-                    int e = core::get_eval(jnd, locked, S.alfrot, S.betrot, S.lambda, S.res, dws);
-                    if (e) {
-                        S.ctl[cFlag] = e;
-                    } else {
+                    flag = warp::get_eval(jnd, locked, S.alfrot, S.betrot, S.lambda, S.res, false, dws, lane);
+                    if (lane == 0 && !flag) {
                         core::convergence_test(jnd, S.lambda, S.res, info, S.wrk2);
                         if (info->nec < info->ned && info->nec > 0) {
                             next_test = (int)((double)(info->ned * info->matvec) / (double)info->nec);
@@ -619,12 +622,12 @@ __device__ void solve(const Params &P, int pid, const Grp &G, double *dyn, long 
                             next_test = next_test + next_test;
                             if (info->maxlan == info->ntot) next_test = (int)ceil(0.5 * (info->maxlan + info->matvec));
                         }
-                        S.ctl[cFlag] = 0;
                     }
-                } else {
-                    S.ctl[cFlag] = 0;
                 }
-                S.ctl[cIter] = next_test;
+                if (lane == 0) {
+                    S.ctl[cFlag] = flag;
+                    S.ctl[cIter] = next_test;
+                }
             }
             G.sync();
             next_test = S.ctl[cIter];
@@ -645,16 +648,21 @@ __device__ void solve(const Params &P, int pid, const Grp &G, double *dyn, long 
             const int jml = jnd - locked;
             int i2 = kept - locked + 1;
             int kk = kept;
+            // One eigen-solve of the tridiagonal serves the test and, at a
+            // restart, the Ritz vectors: with rot applied to them they are
+            // the vectors of the arrowhead matrix too (trl_get_tvec and
+            // trl_get_tvec_a solve it again, each in its own form).
+            bool solved = info->nec < info->ned;
+            if (solved) {
+                st = warp::get_eval(jnd, locked, S.alfrot, S.betrot, S.lambda, S.res, true, dws, lane);
+                if (lane == 0 && !st) core::convergence_test(jnd, S.lambda, S.res, info, S.wrk2);
+                __syncwarp();
+            }
             if (lane == 0) {
-                if (info->nec < info->ned) {
-                    st = core::get_eval(jnd, locked, S.alfrot, S.betrot, S.lambda, S.res, dws);
-                    if (!st) core::convergence_test(jnd, S.lambda, S.res, info, S.wrk2);
-                }
                 if (!st && info->nec < info->ned && info->matvec < info->maxmv) {
                     go = 1;
                     core::shuffle_eig(jml, info->klan - locked, &S.lambda[locked], &S.res[locked], info, &kk,
                                       locked);
-                    path = kk * 3 < jml ? 1 : 2;
                 } else if (!st) {
                     // Final: sort and compute the wanted eigenvectors.
                     kk = min(info->nec, max(info->ned, mev - 1));
@@ -672,23 +680,11 @@ __device__ void solve(const Params &P, int pid, const Grp &G, double *dyn, long 
             __syncwarp();
             int ts = 0;
             if (!st && go) {
-                if (path == 1) {
-                    ts = warp::get_tvec(jml, &S.alfrot[locked], &S.betrot[locked], 0, i2, rot, kk, &S.lambda[locked],
-                                        yy, dws, lane);
-                    if (ts == 0 && lane == 0)
-                        for (int i = 0; i < locked + kk; ++i) S.alpha[i] = S.lambda[i];
-                    __syncwarp();
-                }
-                if (path == 2 || ts != 0) {
-                    if (lane == 0)
-                        for (int i = 0; i < locked + kk; ++i) S.alfrot[i] = S.lambda[i];
-                    __syncwarp();
-                    ts = warp::get_tvec_a(jml, prek - locked, &S.alpha[locked], &S.beta[locked], kk,
-                                          &S.alfrot[locked], yy, dws, lane);
-                }
+                warp::tvec_from(jml, 0, i2, rot, kk, &S.lambda[locked], yy, dws, lane);
+                for (int i = lane; i < locked + kk; i += 32) S.alpha[i] = S.lambda[i];
+                __syncwarp();
                 if (lane == 0) {
-                    if (ts) st = ts;
-                    if (!st) {
+                    {
                         for (int i = 0; i < kk; ++i) S.beta[locked + i] = yy[(size_t)(i + 1) * jml - 1] * S.betrot[jnd - 1];
                         if (jml > info->ned + (info->ned / 5 + 6))
                             core::set_locking(jml, kk, &S.alpha[locked], &S.beta[locked], yy, info->anrm, &i2);

@@ -1,14 +1,16 @@
 // Warp-parallel forms of the small dense routines the batched solver runs at
 // every restart (host/dense_core.h): implicit QL with eigenvector
 // accumulation, Householder tridiagonalisation with Q, the symmetric
-// eigen-solve built on them, and trl_get_tvec / trl_get_tvec_a /
-// trl_tridiag.  All 32 lanes of one warp call them with their lane index.
-// Every element is computed with the same operations in the same order as
-// the serial code, so the results are bitwise those of dense_core.h; only
-// independent rows or columns are spread over the lanes:
-//   * QL: each lane keeps private copies of d and e and runs the (cheap)
-//     scalar bulge chase redundantly; the plane rotations are applied to the
-//     lane's own rows of Z (rows k = lane, lane + 32, ...);
+// eigen-solve built on them, and trl_get_eval / trl_get_tvec /
+// trl_get_tvec_a / trl_tridiag.  All 32 lanes of one warp call them with
+// their lane index.  The algorithms are those of the serial code:
+//   * QL: every lane runs the scalar bulge chase on the shared d and e (lane
+//     0 writes them) and applies the plane rotations to its own rows of Z
+//     (rows k = lane, lane + 32, ...).  The chase is one dependent chain, so
+//     it decides the time: a rotation takes one reciprocal square root and a
+//     correction instead of hypot and two divisions, its inputs are loaded
+//     one rotation ahead, the column shared by two rotations stays in a
+//     register, and the negligible off-diagonal is found by all lanes;
 //   * Householder: p = tau A v by rows, the rank-2 update by columns, Q by
 //     columns; the reflector scalars are computed redundantly.
 // Shared arrays written by one lane and read by others are separated by
@@ -25,76 +27,107 @@ namespace warp {
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kMaxN = 66;  // largest projected problem (maxlan + 2)
 
+// (c, s) = (g, f) / r with r = |(f, g)|; false when r is zero.
+__device__ __forceinline__ bool rotation(double f, double g, double &r, double &s, double &c) {
+    const double r2 = fma(f, f, g * g);
+    if (r2 > 1e-280 && r2 < 1e280) {
+        const double ir = rsqrt(r2);
+        r = r2 * ir;
+        s = f * ir;
+        c = g * ir;
+        // s^2 + c^2 is 1 to a few roundings: one step towards 1.
+        const double t = 0.5 * fma(-s, s, fma(-c, c, 1.0));
+        s = fma(t, s, s);
+        c = fma(t, c, c);
+        return true;
+    }
+    r = hypot(f, g);
+    if (r == 0.0) return false;
+    s = f / r;
+    c = g / r;
+    return true;
+}
+
 __device__ inline int tql_implicit(int n, double *d, double *e, double *Z, int ldz, int zrows, int lane) {
     if (n <= 1) return 0;
-    double dl[kMaxN], el[kMaxN];
-    for (int i = 0; i < n; ++i) {
-        dl[i] = d[i];
-        el[i] = e[i];
-    }
-    el[n - 1] = 0.0;
+    constexpr int RZ = (kMaxN + 31) / 32;  // rows of Z per lane
+    if (lane == 0) e[n - 1] = 0.0;
+    __syncwarp();
     const int max_sweeps = 60;
-    int err = 0;
-    for (int l = 0; l < n && !err; ++l) {
+    for (int l = 0; l < n; ++l) {
         int sweeps = 0;
         for (;;) {
-            int m = l;
-            for (; m < n - 1; ++m) {
-                double dd = fabs(dl[m]) + fabs(dl[m + 1]);
-                if (fabs(el[m]) <= DBL_EPSILON * dd) break;
+            int m = n - 1;
+            for (int b = l; b < n - 1; b += 32) {
+                const int q = b + lane;
+                const bool tiny = q < n - 1 && fabs(e[q]) <= DBL_EPSILON * (fabs(d[q]) + fabs(d[q + 1]));
+                const unsigned found = __ballot_sync(kFull, tiny);
+                if (found) {
+                    m = b + __ffs(found) - 1;
+                    break;
+                }
             }
             if (m == l) break;
-            if (++sweeps > max_sweeps) {
-                err = l + 1;
-                break;
-            }
-            double g = (dl[l + 1] - dl[l]) / (2.0 * el[l]);
+            if (++sweeps > max_sweeps) return l + 1;
+            double g = (d[l + 1] - d[l]) / (2.0 * e[l]);
             double r = hypot(g, 1.0);
-            g = dl[m] - dl[l] + el[l] / (g + (g >= 0.0 ? r : -r));
+            g = d[m] - d[l] + e[l] / (g + (g >= 0.0 ? r : -r));
             double s = 1.0, c = 1.0, p = 0.0;
+            double ei = e[m - 1], di = d[m - 1], d1 = d[m];
+            double zt[RZ];  // this lane's rows of column i + 1
+#pragma unroll
+            for (int u = 0; u < RZ; ++u) {
+                const int k = lane + 32 * u;
+                zt[u] = k < zrows ? Z[(size_t)m * ldz + k] : 0.0;
+            }
+            __syncwarp();  // the chase below rewrites what was read here
             bool deflated = false;
-            for (int i = m - 1; i >= l; --i) {
-                double f = s * el[i];
-                double b = c * el[i];
-                r = hypot(f, g);
-                el[i + 1] = r;
-                if (r == 0.0) {
-                    dl[i + 1] -= p;
-                    el[m] = 0.0;
+            int i = m - 1;
+            for (; i >= l; --i) {
+                const double en = i > l ? e[i - 1] : 0.0, dn = i > l ? d[i - 1] : 0.0;
+                const double f = s * ei, b = c * ei;
+                const bool fine = rotation(f, g, r, s, c);
+                if (lane == 0) e[i + 1] = r;
+                if (!fine) {
                     deflated = true;
                     break;
                 }
-                s = f / r;
-                c = g / r;
-                g = dl[i + 1] - p;
-                r = (dl[i] - g) * s + 2.0 * c * b;
+                g = d1 - p;
+                r = (di - g) * s + 2.0 * c * b;
                 p = s * r;
-                dl[i + 1] = g + p;
+                if (lane == 0) d[i + 1] = g + p;
                 g = c * r - b;
-                if (Z) {
-                    double *zi = Z + (size_t)i * ldz;
-                    double *zi1 = Z + (size_t)(i + 1) * ldz;
-                    for (int k = lane; k < zrows; k += 32) {
-                        double t = zi1[k];
-                        zi1[k] = s * zi[k] + c * t;
-                        zi[k] = c * zi[k] - s * t;
+#pragma unroll
+                for (int u = 0; u < RZ; ++u) {
+                    const int k = lane + 32 * u;
+                    if (k < zrows) {
+                        const double zi = Z[(size_t)i * ldz + k];
+                        Z[(size_t)(i + 1) * ldz + k] = s * zi + c * zt[u];
+                        zt[u] = c * zi - s * zt[u];
                     }
                 }
+                d1 = di;
+                di = dn;
+                ei = en;
             }
-            if (deflated) continue;
-            dl[l] -= p;
-            el[l] = g;
-            el[m] = 0.0;
+#pragma unroll
+            for (int u = 0; u < RZ; ++u) {
+                const int k = lane + 32 * u;
+                if (k < zrows) Z[(size_t)(i + 1) * ldz + k] = zt[u];
+            }
+            if (lane == 0) {
+                if (deflated) {
+                    d[i + 1] -= p;
+                } else {
+                    d[l] -= p;
+                    e[l] = g;
+                }
+                e[m] = 0.0;
+            }
+            __syncwarp();
         }
     }
-    __syncwarp();
-    if (lane == 0)
-        for (int i = 0; i < n; ++i) {
-            d[i] = dl[i];
-            e[i] = el[i];
-        }
-    __syncwarp();
-    return err;
+    return 0;
 }
 
 __device__ inline void tridiag_upper(int n, double *A, int lda, double *d, double *e, bool want_q, double *ws,
@@ -225,12 +258,45 @@ __device__ inline int arrow_to_tridiag(int nd, const double *alpha, const double
     return 0;
 }
 
-__device__ inline int get_tvec(int nd, const double *alpha, const double *beta, int irot, int nrot,
-                               const double *rot, int nlam, const double *lambda, double *yy, double *ws, int lane) {
-    if (nlam <= 0) return 0;
-    double *d = ws, *e = ws + nd, *Z = e + nd, *tmp = Z + (size_t)nd * nd;
-    int *idx = reinterpret_cast<int *>(tmp + nd);
-    char *used = reinterpret_cast<char *>(idx + nlam);
+// core::match_values without a tolerance: every wanted value takes the
+// nearest computed one not yet taken (the first of equals).
+__device__ inline void match_nearest(int n, const double *w, int nlam, const double *lam, int *idx, int lane) {
+    constexpr int R = (kMaxN + 31) / 32;
+    unsigned used = 0;  // of this lane's values lane + 32 u
+    for (int i = 0; i < nlam; ++i) {
+        double bd = 0.0;
+        int best = n;
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+            const int j = lane + 32 * u;
+            if (j < n && !(used >> u & 1)) {
+                const double dd = fabs(w[j] - lam[i]);
+                if (best == n || dd < bd) {
+                    best = j;
+                    bd = dd;
+                }
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double od = __shfl_xor_sync(kFull, bd, o);
+            const int ob = __shfl_xor_sync(kFull, best, o);
+            if (ob < n && (best == n || od < bd || (od == bd && ob < best))) {
+                best = ob;
+                bd = od;
+            }
+        }
+        if (best < n && (best & 31) == lane) used |= 1u << (best >> 5);
+        if (lane == 0) idx[i] = best;
+    }
+    __syncwarp();
+}
+
+// Eigen-solve of the tridiagonal (alpha, beta) of size nd: eigenvalues
+// (unordered) in ws[0 .. nd), their vectors in the columns of
+// ws[2 nd .. 2 nd + nd^2).
+__device__ inline int tridiag_eig(int nd, const double *alpha, const double *beta, double *ws, int lane) {
+    double *d = ws, *e = ws + nd, *Z = e + nd;
     for (int i = lane; i < nd; i += 32) {
         d[i] = alpha[i];
         e[i] = (i + 1 < nd) ? beta[i] : 0.0;
@@ -239,9 +305,46 @@ __device__ inline int get_tvec(int nd, const double *alpha, const double *beta, 
     __syncwarp();
     for (int i = lane; i < nd; i += 32) Z[(size_t)i * nd + i] = 1.0;
     __syncwarp();
-    if (tql_implicit(nd, d, e, Z, nd, nd, lane)) return -132;
-    if (lane == 0) core::match_values(nd, d, nlam, lambda, -1.0, idx, used);
+    return tql_implicit(nd, d, e, Z, nd, nd, lane);
+}
+
+// trl_get_eval; with `vectors` the eigenvectors stay in ws (tridiag_eig) for
+// tvec_from, else only their last components are formed.
+__device__ inline int get_eval(int nd, int locked, const double *alpha, const double *beta, double *lambda,
+                               double *res, bool vectors, double *ws, int lane) {
+    const int m = nd - locked;
+    double *d = ws, *e = ws + m, *Z = e + m;
+    if (vectors) {
+        if (tridiag_eig(m, alpha + locked, beta + locked, ws, lane)) return -122;
+    } else {
+        for (int i = lane; i < m; i += 32) {
+            d[i] = alpha[locked + i];
+            e[i] = (i + 1 < m) ? beta[locked + i] : 0.0;
+            Z[i] = i == m - 1 ? 1.0 : 0.0;
+        }
+        __syncwarp();
+        if (tql_implicit(m, d, e, Z, 1, 1, lane)) return -122;
+    }
+    for (int i = lane; i < nd; i += 32) {
+        lambda[i] = i < locked ? alpha[i] : d[i - locked];
+        res[i] = i < locked ? 0.0 : (vectors ? Z[(size_t)(i - locked) * m + m - 1] : Z[i - locked]);
+    }
     __syncwarp();
+    if (lane == 0) core::sort2(m, lambda + locked, res + locked);
+    __syncwarp();
+    for (int i = locked + lane; i < nd; i += 32) res[i] = beta[nd - 1] * fabs(res[i]);
+    __syncwarp();
+    return 0;
+}
+
+// The eigenvectors of the wanted values lambda from a tridiag_eig in ws, back
+// in the basis before the arrow-to-tridiagonal rotation rot (nrot columns
+// from irot on).
+__device__ inline void tvec_from(int nd, int irot, int nrot, const double *rot, int nlam, const double *lambda,
+                                 double *yy, double *ws, int lane) {
+    double *d = ws, *Z = ws + 2 * nd, *tmp = Z + (size_t)nd * nd;
+    int *idx = reinterpret_cast<int *>(tmp + nd);
+    match_nearest(nd, d, nlam, lambda, idx, lane);
     for (int i = 0; i < nlam; ++i)
         for (int r = lane; r < nd; r += 32) yy[(size_t)i * nd + r] = Z[(size_t)idx[i] * nd + r];
     __syncwarp();
@@ -258,6 +361,13 @@ __device__ inline int get_tvec(int nd, const double *alpha, const double *beta, 
             __syncwarp();
         }
     }
+}
+
+__device__ inline int get_tvec(int nd, const double *alpha, const double *beta, int irot, int nrot,
+                               const double *rot, int nlam, const double *lambda, double *yy, double *ws, int lane) {
+    if (nlam <= 0) return 0;
+    if (tridiag_eig(nd, alpha, beta, ws, lane)) return -132;
+    tvec_from(nd, irot, nrot, rot, nlam, lambda, yy, ws, lane);
     return 0;
 }
 
