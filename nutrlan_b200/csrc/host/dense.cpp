@@ -3,10 +3,11 @@
 // a per-thread workspace.
 #include "dense.h"
 
-#include <complex>
+#include <algorithm>
+#include <cfloat>
 #include <cmath>
-#include <vector>
-
+#include <complex>
+#include <cstring>
 #include <vector>
 
 #include "dense_core.h"
@@ -117,6 +118,133 @@ int arrow_to_tridiag(int nd, const double *alpha, const double *beta, double *ro
 int get_eval(int nd, int locked, const double *alpha, const double *beta, double *lambda, double *res) {
     return core::get_eval(nd, locked, alpha, beta, lambda, res, workspace(nd));
 }
+
+namespace {
+
+constexpr int kRowBlock = 32;  // rows of Z carried through a sweep in registers
+typedef double Rows8 __attribute__((vector_size(64), aligned(8)));
+
+// One QL sweep's rotations (of columns i, i + 1 for i = m - 1 .. l) applied to
+// Z, a block of rows at a time: the column shared by two rotations stays in
+// registers, so a rotation reads and writes one column.  Four vectors of
+// eight rows cover the latency of a rotation's dependent multiply and add
+// (two took 2.0 ms where four take 1.1, at 128 columns).  ld is a multiple of
+// the block.
+__attribute__((target_clones("avx512f", "avx2", "default"))) void apply_sweep(int l, int m, const double *cs,
+                                                                              const double *sn, double *Z, int ld) {
+    constexpr int V = kRowBlock / 8;
+    for (int r0 = 0; r0 < ld; r0 += kRowBlock) {
+        Rows8 t[V];
+        Rows8 *z = reinterpret_cast<Rows8 *>(Z + (size_t)m * ld + r0);
+        for (int k = 0; k < V; ++k) t[k] = z[k];
+        for (int i = m - 1; i >= l; --i) {
+            const double c = cs[i], s = sn[i];
+            Rows8 *zi = reinterpret_cast<Rows8 *>(Z + (size_t)i * ld + r0);
+            Rows8 *zi1 = reinterpret_cast<Rows8 *>(Z + (size_t)(i + 1) * ld + r0);
+            for (int k = 0; k < V; ++k) {
+                const Rows8 v = zi[k];
+                zi1[k] = s * v + c * t[k];
+                t[k] = c * v - s * t[k];
+            }
+        }
+        z = reinterpret_cast<Rows8 *>(Z + (size_t)l * ld + r0);
+        for (int k = 0; k < V; ++k) z[k] = t[k];
+    }
+}
+
+}  // namespace
+
+// core::tql_implicit with the rotations of a sweep recorded and applied to Z
+// together.
+int TridiagVectors::get_eval(int nd, int locked, const double *alpha, const double *beta, double *lambda,
+                             double *res) {
+    const int n = nd - locked;
+    n_ = n;
+    ld_ = (n + kRowBlock - 1) / kRowBlock * kRowBlock;
+    d_.assign(alpha + locked, alpha + nd);
+    e_.assign(n, 0.0);
+    for (int i = 0; i + 1 < n; ++i) e_[i] = beta[locked + i];
+    Z_.assign((size_t)ld_ * n, 0.0);
+    for (int i = 0; i < n; ++i) Z_[(size_t)i * ld_ + i] = 1.0;
+    cs_.resize(n);
+    sn_.resize(n);
+    double *d = d_.data(), *e = e_.data();
+    const int max_sweeps = 60;
+    for (int l = 0; l < n; ++l) {
+        int sweeps = 0;
+        for (;;) {
+            int m = l;
+            for (; m < n - 1; ++m) {
+                const double dd = std::fabs(d[m]) + std::fabs(d[m + 1]);
+                if (std::fabs(e[m]) <= DBL_EPSILON * dd) break;
+            }
+            if (m == l) break;
+            if (++sweeps > max_sweeps) return -122;
+            double g = (d[l + 1] - d[l]) / (2.0 * e[l]);
+            double r = std::hypot(g, 1.0);
+            g = d[m] - d[l] + e[l] / (g + (g >= 0.0 ? r : -r));
+            double s = 1.0, c = 1.0, p = 0.0;
+            int i = m - 1;
+            bool deflated = false;
+            for (; i >= l; --i) {
+                const double f = s * e[i], b = c * e[i];
+                const bool turned = core::plane_rotation(f, g, &r, &s, &c);
+                e[i + 1] = r;
+                if (!turned) {
+                    d[i + 1] -= p;
+                    e[m] = 0.0;
+                    deflated = true;
+                    break;
+                }
+                g = d[i + 1] - p;
+                r = (d[i] - g) * s + 2.0 * c * b;
+                p = s * r;
+                d[i + 1] = g + p;
+                g = c * r - b;
+                cs_[i] = c;
+                sn_[i] = s;
+            }
+            apply_sweep(i + 1, m, cs_.data(), sn_.data(), Z_.data(), ld_);
+            if (deflated) continue;
+            d[l] -= p;
+            e[l] = g;
+            e[m] = 0.0;
+        }
+    }
+    for (int i = 0; i < locked; ++i) {
+        lambda[i] = alpha[i];
+        res[i] = 0.0;
+    }
+    for (int i = 0; i < n; ++i) {
+        lambda[locked + i] = d[i];
+        res[locked + i] = Z_[(size_t)i * ld_ + n - 1];
+    }
+    core::sort2(n, lambda + locked, res + locked);
+    for (int i = locked; i < nd; ++i) res[i] = beta[nd - 1] * std::fabs(res[i]);
+    return 0;
+}
+
+void TridiagVectors::vectors(int nrot, const double *rot, int nlam, const double *lambda, double *yy) const {
+    if (nlam <= 0) return;
+    std::vector<int> idx(nlam);
+    std::vector<char> used(n_);
+    std::vector<double> tmp(std::max(nrot, 1));
+    core::match_values(n_, d_.data(), nlam, lambda, -1.0, idx.data(), used.data());
+    for (int c = 0; c < nlam; ++c) {
+        double *col = yy + (size_t)c * n_;
+        std::memcpy(col, Z_.data() + (size_t)idx[c] * ld_, sizeof(double) * n_);
+        if (nrot > 1) {
+            std::fill(tmp.begin(), tmp.end(), 0.0);
+            for (int k = 0; k < nrot; ++k) {
+                const double w = col[k];
+                const double *rk = rot + (size_t)k * nrot;
+                for (int i = 0; i < nrot; ++i) tmp[i] += rk[i] * w;
+            }
+            std::memcpy(col, tmp.data(), sizeof(double) * nrot);
+        }
+    }
+}
+
 int get_tvec(int nd, const double *alpha, const double *beta, int irot, int nrot, const double *rot, int nlam,
              const double *lambda, double *yy) {
     return core::get_tvec(nd, alpha, beta, irot, nrot, rot, nlam, lambda, yy, workspace(nd));

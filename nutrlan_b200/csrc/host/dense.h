@@ -64,6 +64,23 @@ int arrow_to_tridiag(int nd, const double *alpha, const double *beta,
 int get_eval(int nd, int locked, const double *alpha, const double *beta,
              double *lambda, double *res);
 
+// The same with the eigenvectors kept: one solve of the tridiagonal serves the
+// convergence test and the Ritz vectors of the restart or result after it
+// (trl_get_tvec and trl_get_tvec_a solve the projected problem again, each in
+// its own form; these vectors are theirs up to sign and rounding).
+class TridiagVectors {
+   public:
+    int get_eval(int nd, int locked, const double *alpha, const double *beta, double *lambda, double *res);
+    // For the wanted values lambda[0..nlam): yy (nd x nlam, nd = size of the
+    // solved problem), with rot (nrot x nrot) applied to the first nrot rows.
+    void vectors(int nrot, const double *rot, int nlam, const double *lambda, double *yy) const;
+    int size() const { return n_; }
+
+   private:
+    int n_ = 0, ld_ = 0;
+    std::vector<double> d_, e_, Z_, cs_, sn_;
+};
+
 // trl_get_tvec: eigenvectors of the tridiagonal (alpha, beta) for the given
 // Ritz values lambda[0..nlam), then rot (nrot x nrot) applied to rows
 // irot..irot+nrot of each vector.  yy is nd x nlam.

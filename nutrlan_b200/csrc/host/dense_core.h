@@ -153,11 +153,15 @@ TRLB_HD inline void tridiag_upper(int n, double *A, int lda, double *d, double *
         taus[k] = tau;
         e[k - 1] = beta;
         // Two-sided update of the leading k x k block: A <- H A H.
-        for (int i = 0; i < k; ++i) {
-            double s = 0.0;
-            for (int j = 0; j < k; ++j) s += a(i, j) * v[j];
-            p[i] = tau * s;
+        // (p by columns and Q below by blocks of columns: contiguous or
+        // independent sums, each in the order of its index)
+        for (int i = 0; i < k; ++i) p[i] = 0.0;
+        for (int j = 0; j < k; ++j) {
+            const double vj = v[j];
+            const double *aj = A + (size_t)j * lda;
+            for (int i = 0; i < k; ++i) p[i] += aj[i] * vj;
         }
+        for (int i = 0; i < k; ++i) p[i] *= tau;
         double pv = 0.0;
         for (int i = 0; i < k; ++i) pv += p[i] * v[i];
         for (int i = 0; i < k; ++i) w[i] = p[i] - 0.5 * tau * pv * v[i];
@@ -181,13 +185,35 @@ TRLB_HD inline void tridiag_upper(int n, double *A, int lda, double *d, double *
         double tau = taus[k];
         if (tau == 0.0) continue;
         const double *v = &vs[(size_t)k * n];
-        for (int j = 0; j < n; ++j) {
-            double s = 0.0;
-            for (int i = 0; i < k; ++i) s += v[i] * a(i, j);
-            s *= tau;
-            for (int i = 0; i < k; ++i) a(i, j) -= s * v[i];
+        constexpr int NB = 8;
+        for (int j0 = 0; j0 < n; j0 += NB) {
+            const int nb = hmin(NB, n - j0);
+            double s[NB] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            if (nb == NB) {
+                for (int i = 0; i < k; ++i)
+                    for (int q = 0; q < NB; ++q) s[q] += v[i] * a(i, j0 + q);
+            } else {
+                for (int q = 0; q < nb; ++q)
+                    for (int i = 0; i < k; ++i) s[q] += v[i] * a(i, j0 + q);
+            }
+            for (int q = 0; q < nb; ++q) {
+                const double sq = s[q] * tau;
+                double *aj = A + (size_t)(j0 + q) * lda;
+                for (int i = 0; i < k; ++i) aj[i] -= sq * v[i];
+            }
         }
     }
+}
+
+// (c, s) = (g, f) / r with r = |(f, g)|; false when r is zero.  The squares
+// are scaled (hypot) only where they could leave the range of a double.
+TRLB_HD inline bool plane_rotation(double f, double g, double *r, double *s, double *c) {
+    const double r2 = f * f + g * g;
+    *r = r2 > 1e-280 && r2 < 1e280 ? sqrt(r2) : hypot(f, g);
+    if (*r == 0.0) return false;
+    *s = f / *r;
+    *c = g / *r;
+    return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -218,16 +244,14 @@ TRLB_HD inline int tql_implicit(int n, double *d, double *e, double *Z, int ldz,
             for (int i = m - 1; i >= l; --i) {
                 double f = s * e[i];
                 double b = c * e[i];
-                r = hypot(f, g);
+                const bool turned = plane_rotation(f, g, &r, &s, &c);
                 e[i + 1] = r;
-                if (r == 0.0) {
+                if (!turned) {
                     d[i + 1] -= p;
                     e[m] = 0.0;
                     deflated = true;
                     break;
                 }
-                s = f / r;
-                c = g / r;
                 g = d[i + 1] - p;
                 r = (d[i] - g) * s + 2.0 * c * b;
                 p = s * r;

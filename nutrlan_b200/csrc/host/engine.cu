@@ -404,6 +404,7 @@ class Engine {
 
     // host state (reference names)
     std::vector<double> alpha_, beta_, alfrot_, betrot_, rot_, lambda_, res_, yy_, wrk2_;
+    TridiagVectors tridiag_;
     int final_j1_ = 0;
     double ritz_min_ = 1e300, ritz_max_ = -1e300;  // extreme Ritz values seen (spectrum bounds)
     long long launches_ = 0;
@@ -1777,29 +1778,18 @@ void Engine<T>::run() {
         prek = kept;
         const int jml = jnd - locked;
         int i2 = kept - locked + 1;
-        if (info->nec < info->ned) {
-            if ((stat = get_eval(jnd, locked, alfrot_.data(), betrot_.data(), lambda_.data(), res_.data()))) break;
+        const bool solved = info->nec < info->ned;
+        if (solved) {
+            if ((stat = tridiag_.get_eval(jnd, locked, alfrot_.data(), betrot_.data(), lambda_.data(), res_.data())))
+                break;
             track_ritz(jnd);
             convergence_test(jnd, lambda_.data(), res_.data(), info, wrk2_.data());
             log_progress();
         }
         if (info->nec < info->ned && info->matvec < info->maxmv) {
             shuffle_eig(jml, info->klan - locked, &lambda_[locked], &res_[locked], info, &kept, locked);
-            int tstat = 0;
-            if (kept * 3 < jml) {
-                tstat = get_tvec(jml, &alfrot_[locked], &betrot_[locked], 0, i2, rot_.data(), kept, &lambda_[locked],
-                                 yy_.data());
-                if (tstat == 0 && locked + kept > 0) std::memcpy(alpha_.data(), lambda_.data(), sizeof(double) * (locked + kept));
-            }
-            if (kept * 3 >= jml || tstat != 0) {
-                if (locked + kept > 0) std::memcpy(alfrot_.data(), lambda_.data(), sizeof(double) * (locked + kept));
-                tstat = get_tvec_a(jml, prek - locked, &alpha_[locked], &beta_[locked], kept, &alfrot_[locked],
-                                   yy_.data());
-            }
-            if (tstat) {
-                stat = tstat;
-                break;
-            }
+            tridiag_.vectors(i2, rot_.data(), kept, &lambda_[locked], yy_.data());
+            if (locked + kept > 0) std::memcpy(alpha_.data(), lambda_.data(), sizeof(double) * (locked + kept));
             for (int i = 0; i < kept; ++i) beta_[locked + i] = yy_[(size_t)(i + 1) * jml - 1] * betrot_[jnd - 1];
             if (jml > info->ned + (info->ned / 5 + 6))
                 set_locking(jml, kept, &alpha_[locked], &beta_[locked], yy_.data(), info->anrm, &i2);
@@ -1845,9 +1835,11 @@ void Engine<T>::run() {
             sort_eig(jnd, info->lohi, kept, info->ref, lambda_.data(), res_.data());
             std::memcpy(eval_, lambda_.data(), sizeof(double) * kept);
             int tstat = 0;
-            if (kept * 3 < jnd)
+            if (solved && locked == 0)
+                tridiag_.vectors(i2, rot_.data(), kept, eval_, yy_.data());
+            else if (kept * 3 < jnd)
                 tstat = get_tvec(jnd, alfrot_.data(), betrot_.data(), locked, i2, rot_.data(), kept, eval_, yy_.data());
-            if (kept * 3 >= jnd || tstat != 0) {
+            if ((!(solved && locked == 0) && kept * 3 >= jnd) || tstat != 0) {
                 tstat = get_tvec_a(jnd, prek, alpha_.data(), beta_.data(), kept, eval_, yy_.data());
                 if (tstat) {
                     stat = tstat;

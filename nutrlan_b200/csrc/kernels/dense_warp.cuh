@@ -287,7 +287,7 @@ __device__ inline void match_nearest(int n, const double *w, int nlam, const dou
             }
         }
         if (best < n && (best & 31) == lane) used |= 1u << (best >> 5);
-        if (lane == 0) idx[i] = best;
+        if (lane == 0) idx[i] = best < n ? best : 0;  // (no value left only if one is not a number)
     }
     __syncwarp();
 }
