@@ -262,8 +262,12 @@ __device__ inline double reduce_columns(const C *part, int nb, int m, C *out, C 
             smem[threadIdx.x] = s;  // keep for the norm below
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int g = 0; g < groups && c0 + g < m; ++g) norm2 += abs2(smem[g * tpc]);
+        if (threadIdx.x < 32) {  // by the first warp: one thread alone waits for each in turn
+            double s = 0.0;
+            for (int g = threadIdx.x; g < groups && c0 + g < m; g += 32) s += abs2(smem[g * tpc]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += shfl_down(s, o);
+            norm2 += s;
         }
         __syncthreads();
     }

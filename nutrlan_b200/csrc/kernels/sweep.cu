@@ -22,7 +22,7 @@
 //
 // Bound by memory; measured against the two kernels and the normalisation
 // (one B200): 256^3 FP64, 128 steps, 427 -> 280 ms a call; 1024^2
-// complex128, 64.3 -> 41.7 ms; 101^3 FP32, 30.3 -> 18.0 ms; 2048^2
+// complex128, 64.3 -> 39.3 ms; 101^3 FP32, 30.3 -> 17.5 ms; 2048^2
 // complex64, 80.0 -> 68.7 ms (12 FP64 FMAs and two conversions per 8 bytes:
 // the sweep itself runs at 3.0-3.5 TB/s there, 5.1-5.7 for FP64 storage).
 //
@@ -352,16 +352,57 @@ __global__ void __launch_bounds__(kNT, 1) k_sweep(const SweepArgs<T> A, long chu
         part_r2[blockIdx.x] = rs;
     }
     if (!last_block_arrived(ticket)) return;
-    C *const tot = reinterpret_cast<C *>(smem);
-    const double h2 = reduce_columns(part, (int)gridDim.x, m, A.a, tot);
+    // Totals, T h and the scalars, one column per thread (k + 1 <= 129 of
+    // them).  A thread's loads are all in flight at once; with eight at a
+    // time, and one thread alone for |h|^2 and for the coupled row, every
+    // sweep took 7 to 30 us longer (FP64, 2^21 rows, 4 and 128 columns: 35.8
+    // and 437.8 -> 28.1 and 410.0 us; 64^3 FP64 13.5 -> 12.2 ms a call).
+    const int per = kNT / m, col = tid % m, part_of = tid / m;
+    // Row tid of T: diagonal, coupling to the next and to the last column
+    // (the new entries are stored below).
+    const double bprev = sqrt(b2);
+    auto tb = [&](int i) { return i == k - 1 && !A.first ? bprev : A.tb[i]; };
+    const double ti = tid < k ? A.ta[tid] : alpha, bi = tid < k ? tb(tid) : 0.0;
+    const double bl = tid >= 1 && tid <= k ? tb(tid - 1) : 0.0;
+    C sum = czero(C());
+    if (part_of < per) {
+        constexpr int U = 32;
+        for (int b0 = part_of; b0 < (int)gridDim.x; b0 += U * per) {
+            C v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int b = b0 + u * per;
+                v[u] = b < (int)gridDim.x ? ldcg(part + (long)b * m + col) : czero(C());
+            }
+#pragma unroll
+            for (int o = U / 2; o > 0; o >>= 1)
+#pragma unroll
+                for (int u = 0; u < o; ++u) v[u] = v[u] + v[u + o];
+            sum = sum + v[0];
+        }
+    }
+    C *const tot = reinterpret_cast<C *>(smem), *const hs = tot + kNT;
+    tot[tid] = sum;
+    __syncthreads();
+    C hi = czero(C());
+    if (tid < m) {
+        for (int q = 0; q < per; ++q) hi = hi + tot[q * m + tid];
+        A.a[tid] = hi;
+        hs[tid] = hi;
+    }
     const double r2 = sum_partials(part_r2, (int)gridDim.x, red_d);
+    const double h2 = block_sum(abs2(hi), red_d);
+    C arrow = czero(C());
+    if (A.kept > 0) arrow = block_sum(tid < A.kept ? bi * hi : czero(C()), red_s);
     __shared__ double nb2;
+    __shared__ C coupled;
     if (tid == 0) {
         const double b = r2 - h2;
         nb2 = b;
+        coupled = arrow;
         A.ta[k] = alpha;
         if (!A.first) {
-            A.tb[k - 1] = sqrt(b2);
+            A.tb[k - 1] = bprev;
             A.lg_prev[3] = b2;
         }
         A.sc[0] = 1.0 / sqrt(b);
@@ -373,17 +414,17 @@ __global__ void __launch_bounds__(kNT, 1) k_sweep(const SweepArgs<T> A, long chu
         *ticket = 0;
     }
     __syncthreads();
-    for (int i = tid; i <= k; i += kNT) {
-        C s = A.ta[i] * A.a[i];
+    if (tid <= k) {
+        const int i = tid;
+        C s = ti * hi;
         if (i < A.kept) {
-            s = s + A.tb[i] * A.a[A.kept];
+            s = s + bi * hs[A.kept];
         } else {
-            if (i > A.kept) {
-                s = s + A.tb[i - 1] * A.a[i - 1];
-            } else {
-                for (int l = 0; l < A.kept; ++l) s = s + A.tb[l] * A.a[l];
-            }
-            if (i < k) s = s + A.tb[i] * A.a[i + 1];
+            if (i > A.kept)
+                s = s + bl * hs[i - 1];
+            else
+                s = s + coupled;
+            if (i < k) s = s + bi * hs[i + 1];
         }
         if (kWide && i == k) s = s + as_c(nb2, C());
         A.c[i] = s;
