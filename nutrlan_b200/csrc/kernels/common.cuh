@@ -174,6 +174,10 @@ __device__ __forceinline__ void store_c(zd *p, const zd (&o)[R]) {
     for (int k = 0; k < R; ++k) *reinterpret_cast<double2 *>(p + k) = make_double2(o[k].x, o[k].y);
 }
 
+// Lets a kernel launched behind this one for it (sweep.cu) be set up while this
+// one still runs; any other launch waits for the end as always.
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- asynchronous copies into shared memory (16 bytes per thread) -------------
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
     const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);

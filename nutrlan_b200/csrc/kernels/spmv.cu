@@ -47,6 +47,7 @@ __global__ void __launch_bounds__(kThreads)
     k_csr(int nrow, long n_pad, const long long *__restrict__ rp, const int *__restrict__ ci,
           const V *__restrict__ va, const V *__restrict__ x, V *__restrict__ y, double *part,
           unsigned *ticket, double *alpha_out) {
+    next_may_start();
     const int g = threadIdx.x & (kGroup - 1);
     const long groups = (long)gridDim.x * (kThreads / kGroup);
     double aacc = 0.0;
@@ -97,6 +98,7 @@ __global__ void __launch_bounds__(kThreads)
                  unsigned *ticket, double *alpha_out) {
     __shared__ V prod[kChunk];
     __shared__ long long rps[kThreads + 1];
+    next_may_start();
     const int t = threadIdx.x;
     double aacc = 0.0;
     const long ntiles = n_pad / kThreads;
@@ -155,6 +157,7 @@ __global__ void __launch_bounds__(kThreads, 8)
            const int *__restrict__ ci, const V *__restrict__ va, const int *__restrict__ perm,
            const V *__restrict__ x, V *__restrict__ y, double *part, unsigned *ticket,
            double *alpha_out) {
+    next_may_start();
     const int lane = threadIdx.x & 31;
     const long warps = (long)gridDim.x * (kThreads / 32);
     double aacc = 0.0;

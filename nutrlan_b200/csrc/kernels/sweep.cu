@@ -22,8 +22,8 @@
 //
 // Bound by memory; measured against the two kernels and the normalisation
 // (one B200): 256^3 FP64, 128 steps, 427 -> 280 ms a call; 1024^2
-// complex128, 64.3 -> 39.3 ms; 101^3 FP32, 30.3 -> 17.5 ms; 2048^2
-// complex64, 80.0 -> 68.7 ms (12 FP64 FMAs and two conversions per 8 bytes:
+// complex128, 64.3 -> 39.1 ms; 101^3 FP32, 30.3 -> 16.9 ms; 2048^2
+// complex64, 82.4 -> 65.6 ms (12 FP64 FMAs and two conversions per 8 bytes:
 // the sweep itself runs at 3.0-3.5 TB/s there, 5.1-5.7 for FP64 storage).
 //
 // For a 32-bit basis the working vectors stay FP64: q_{k-1} is read from its
@@ -167,12 +167,17 @@ __global__ void __launch_bounds__(kNT, 1) k_sweep(const SweepArgs<T> A, long chu
     int issued = 0;
     unsigned ifill = 0, iuse = 0;  // byte offsets of the stages to fill and to use
     auto next_stage = [](unsigned o) { return o == (unsigned)((NS - 1) * Sh::kStage) ? 0u : o + Sh::kStage; };
-    auto issue = [&]() {
+    auto fill_cols = [&]() {
         if (issued < nit) {
             unsigned char *d = smem + ifill + warp * Sh::kSlot + lane * 16;
 #pragma unroll
             for (int q = 0; q < NC; ++q)
                 if (on(q)) cp_async16(d + q * 512, from + (size_t)off[q] * 16);
+            from += (long)step * (int)sizeof(T);
+        }
+    };
+    auto fill_vecs = [&]() {
+        if (issued < nit) {
             unsigned char *dv = smem + ifill + kWarps * Sh::kSlot + slice * Sh::kVecs * Sh::kVec + lane * 16;
 #pragma unroll
             for (int j = 0; j < kVecCopies; ++j) {
@@ -182,15 +187,35 @@ __global__ void __launch_bounds__(kNT, 1) k_sweep(const SweepArgs<T> A, long chu
                                reinterpret_cast<const char *>(src + vrow) + (j % kPerVec) * 512 + lane * 16);
                 }
             }
-            from += (long)step * (int)sizeof(T);
             vrow += step;
         }
-        cp_async_commit();
+    };
+    auto filled = [&]() {
         ++issued;
         ifill = next_stage(ifill);
     };
+    auto issue = [&]() {
+        fill_cols();
+        fill_vecs();
+        cp_async_commit();
+        filled();
+    };
+    // The kernel may start before the operator's (launch_sweep): the basis is
+    // older than that one, the vectors and the scalars are read after it.
 #pragma unroll
-    for (int t = 0; t < NS - 1; ++t) issue();
+    for (int t = 0; t < NS - 1; ++t) {
+        fill_cols();
+        filled();
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    issued = 0;
+    ifill = 0;
+#pragma unroll
+    for (int t = 0; t < NS - 1; ++t) {
+        fill_vecs();
+        cp_async_commit();
+        filled();
+    }
     const double ib = A.sc[0], b2 = A.sc[1], rbeta = kWide ? 0.0 : A.sc[2];
     const C hl = A.a[k - 1];
     const double alpha = *A.dot / b2 - 2.0 * real_part(hl);
@@ -480,7 +505,20 @@ void launch_sweep(const SweepArgs<T> &a, Scratch &s, cudaStream_t st) {
     const int per = (a.k + (1 << lg) - 1) >> lg;  // columns per group
     const int nc = lg == 0 ? (per <= 8 ? 0 : (per <= 12 ? 1 : 2)) : (std::max(per, 10) - 9) / 2;
     const Variant<T> &v = kern[lg][nc];
-    v.kern<<<nb, kNT, v.smem, st>>>(a, chunk, part, part_r2, s.tickets + kTicketSweep);
+    // Launched while the operator's kernel ends (which lets it at its start;
+    // that one itself starts when the sweep before is complete): 64^3 FP64
+    // 12.2 -> 11.7 ms a call, 101^3 FP32 17.5 -> 16.9 ms.
+    cudaLaunchAttribute early = {};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nb);
+    cfg.blockDim = dim3(kNT);
+    cfg.dynamicSmemBytes = v.smem;
+    cfg.stream = st;
+    cfg.attrs = &early;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, v.kern, a, chunk, part, part_r2, s.tickets + kTicketSweep);
 }
 
 template void launch_sweep<double>(const SweepArgs<double> &, Scratch &, cudaStream_t);
