@@ -1114,8 +1114,8 @@ int Engine<T>::final_vectors(int jnd, int kept) {
 // or more, one cooperative kernel for shorter CSR problems, else the discrete
 // kernels (FP64/c128 basis; a shorter 32-bit basis takes its steps one by
 // one).  Sweeps and the cooperative kernel differ from the sequential path in
-// rounding only.  Measured at 2^18 rows, 128 columns: 25.3 ms a solve with
-// the discrete kernels, 17.2 with sweeps.
+// rounding only.  Measured at 2^18 rows, 128 columns: 25.1 ms a solve with
+// the discrete kernels, 11.7 with sweeps.
 template <class T>
 bool Engine<T>::spec_enabled() const {
     if (!builtin_ || uo_ || comm_ || builtin_->halo) return false;

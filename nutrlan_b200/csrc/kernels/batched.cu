@@ -473,7 +473,9 @@ __device__ inline int orth(const Params &P, int pid, double *V, int ld, int n, i
 // copied (cp.async) while this one is multiplied.  A thread forms four
 // outputs of a row: per column one 8-byte tile read and two 16-byte
 // broadcasts of yy, regrouped by columns, for four multiply-adds; every
-// output sums over c in ascending order.  @@
+// output sums over c in ascending order.  Against one tile at a time and an
+// 8-byte read of yy per multiply-add: 400 problems, grids 48-160, 258 -> 251
+// ms; 40 problems, grids 20-64, 18.3 -> 17.4 ms.
 __device__ inline void ritz_in_place(double *V, int ld, int n, int lck, int jml, int kept, const double *yy,
                                      double *yt, double *tile, long tile_cap /* doubles */, const Grp &G) {
     // Rows per tile: what half the free shared memory holds (maxlan + 4 at
