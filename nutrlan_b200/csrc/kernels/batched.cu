@@ -465,83 +465,56 @@ __device__ inline int orth(const Params &P, int pid, double *V, int ld, int n, i
 }
 
 // In place V[:, lck .. lck+kept) <- V[:, lck .. lck+jml) * yy (jml x kept),
-// tile by tile (the group owns every row, so no other reader exists).  yt:
-// jml x kept doubles of workspace.
-//
-// The basis columns come from memory and the products from shared memory,
-// which is what bounds each of them; two tiles, so that the next one is
-// copied (cp.async) while this one is multiplied.  A thread forms four
-// outputs of a row: per column one 8-byte tile read and two 16-byte
-// broadcasts of yy, regrouped by columns, for four multiply-adds; every
-// output sums over c in ascending order.  Against one tile at a time and an
-// 8-byte read of yy per multiply-add: 400 problems, grids 48-160, 258 -> 251
-// ms; 40 problems, grids 20-64, 18.3 -> 17.4 ms.
+// tile by tile (the CTA owns every row, so no other reader exists).
 __device__ inline void ritz_in_place(double *V, int ld, int n, int lck, int jml, int kept, const double *yy,
-                                     double *yt, double *tile, long tile_cap /* doubles */, const Grp &G) {
-    // Rows per tile: what half the free shared memory holds (maxlan + 4 at
-    // least: the dense workspace is there), in whole warps from 32 on, else
-    // even, for the 16-byte copies.
-    const int half = (int)(tile_cap / 2 / max(jml, 1));
-    const int kTile = half >= 32 ? min(half, n + 31) / 32 * 32 : half / 2 * 2;
-    const int k4 = kept & ~3, items = k4 / 4 + (kept - k4);  // columns in fours, then one by one
-    for (int e = G.tid; e < jml * k4; e += G.nt) {
-        const int c = e / k4, k = e - c * k4;
-        yt[e] = yy[(size_t)k * jml + c];
-    }
-    auto fill = [&](int r0, double *to) {
-        const int rows = min(kTile, n - r0), rp = rows / 2, rest = rows - 2 * rp;
-        for (int e = G.tid; e < rp * jml; e += G.nt) {
-            const int c = e / rp, pr = e - c * rp;
-            cp_async16(to + c * kTile + 2 * pr, V + (size_t)(lck + c) * ld + r0 + 2 * pr);
-        }
-        for (int c = G.tid; c < rest * jml; c += G.nt)  // an odd last row
-            to[c * kTile + 2 * rp] = V[(size_t)(lck + c) * ld + r0 + 2 * rp];
-        cp_async_commit();
-    };
-    double *cur = tile, *next = tile + kTile * jml;
-    fill(0, cur);
+                                     double *tile, long tile_cap /* doubles */, const Grp &G) {
+    // As many rows per tile as the group's free shared memory holds (two
+    // group barriers per tile), rounded down to a multiple of 32 when that
+    // is at least 32; never more than the capacity.
+    int kTile = (int)min((long)n, tile_cap / max(jml, 1));
+    if (kTile >= 32) kTile = kTile / 32 * 32;
+    kTile = max(kTile, 1);
+    // Tile fill: row pairs with 16-byte loads when the tile height is even
+    // (r0, rr even: aligned in the basis column and in the tile).  Products:
+    // each thread forms two output columns from one read of the tile value;
+    // every output sums over c in ascending order.
+    const bool pairs = (kTile & 1) == 0;
+    const int kp = kept / 2;
     for (int r0 = 0; r0 < n; r0 += kTile) {
-        if (r0 + kTile < n) {
-            fill(r0 + kTile, next);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
+        const int rows = min(kTile, n - r0);
+        const int rp = pairs ? rows / 2 : 0;
+        for (int e = G.tid; e < rp * jml; e += G.nt) {
+            const int pr = e % rp, c = e / rp;
+            const double2 v = ld2(V + (size_t)(lck + c) * ld + r0 + 2 * pr);
+            *reinterpret_cast<double2 *>(tile + c * kTile + 2 * pr) = v;
+        }
+        const int rest = rows - 2 * rp;  // rows not covered by pairs
+        for (int e = G.tid; e < rest * jml; e += G.nt) {
+            const int rr = 2 * rp + e % rest, c = e / rest;
+            tile[c * kTile + rr] = V[(size_t)(lck + c) * ld + r0 + rr];
         }
         G.sync();
-        const int rows = min(kTile, n - r0);
-        for (int e = G.tid; e < rows * items; e += G.nt) {
-            const int q = e / rows, rr = e - q * rows;
-            const double *t = cur + rr;
-            if (4 * q < k4) {
-                const double *y = yt + 4 * q;
-                double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-#pragma unroll 4
-                for (int c = 0; c < jml; ++c, y += k4) {
-                    const double v = t[c * kTile];
-                    const double2 ya = ld2(y), yb = ld2(y + 2);
-                    s0 = fma(v, ya.x, s0);
-                    s1 = fma(v, ya.y, s1);
-                    s2 = fma(v, yb.x, s2);
-                    s3 = fma(v, yb.y, s3);
-                }
-                double *o = V + (size_t)(lck + 4 * q) * ld + r0 + rr;
-                o[0] = s0;
-                o[(size_t)ld] = s1;
-                o[2 * (size_t)ld] = s2;
-                o[3 * (size_t)ld] = s3;
-            } else {
-                const int k = k4 + (q - k4 / 4);
-                const double *y = yy + (size_t)k * jml;
+        for (int e = G.tid; e < rows * kp; e += G.nt) {
+            const int rr = e % rows, k = 2 * (e / rows);
+            const double *y0 = yy + (size_t)k * jml, *y1 = y0 + jml;
+            double s0 = 0.0, s1 = 0.0;
+            for (int c = 0; c < jml; ++c) {
+                const double t = tile[c * kTile + rr];
+                s0 = fma(t, y0[c], s0);
+                s1 = fma(t, y1[c], s1);
+            }
+            V[(size_t)(lck + k) * ld + r0 + rr] = s0;
+            V[(size_t)(lck + k + 1) * ld + r0 + rr] = s1;
+        }
+        if (kept & 1) {
+            const int k = kept - 1;
+            for (int rr = G.tid; rr < rows; rr += G.nt) {
                 double s = 0.0;
-#pragma unroll 4
-                for (int c = 0; c < jml; ++c) s = fma(t[c * kTile], y[c], s);
+                for (int c = 0; c < jml; ++c) s = fma(tile[c * kTile + rr], yy[(size_t)k * jml + c], s);
                 V[(size_t)(lck + k) * ld + r0 + rr] = s;
             }
         }
         G.sync();
-        double *const used = cur;
-        cur = next;
-        next = used;
     }
 }
 
@@ -750,7 +723,7 @@ __device__ void solve(const Params &P, int pid, const Grp &G, double *dyn, long 
         kept = S.ctl[cKept];
         if (S.ctl[cGo]) {
             // Restart: kept Ritz vectors in place, then the residual vector.
-            ritz_in_place(V, ld, n, locked, jml, kept, yy, rot, tile, tile_cap, G);
+            ritz_in_place(V, ld, n, locked, jml, kept, yy, tile, tile_cap, G);
             const double *rr = V + (size_t)jnd * ld;
             double *dst = V + (size_t)(locked + kept) * ld;
             for (int i = G.tid; i < n; i += G.nt) dst[i] = rr[i];
