@@ -652,7 +652,8 @@ __device__ void solve(const Params &P, int pid, const Grp &G, double *dyn, long 
             // restart, the Ritz vectors: with rot applied to them they are
             // the vectors of the arrowhead matrix too (trl_get_tvec and
             // trl_get_tvec_a solve it again, each in its own form).
-            bool solved = info->nec < info->ned;
+            const bool solved = info->nec < info->ned;
+            __syncwarp();  // lane 0 sets nec below
             if (solved) {
                 st = warp::get_eval(jnd, locked, S.alfrot, S.betrot, S.lambda, S.res, true, dws, lane);
                 if (lane == 0 && !st) core::convergence_test(jnd, S.lambda, S.res, info, S.wrk2);

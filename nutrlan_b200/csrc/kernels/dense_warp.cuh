@@ -10,7 +10,8 @@
 //     it decides the time: a rotation takes one reciprocal square root and a
 //     correction instead of hypot and two divisions, its inputs are loaded
 //     one rotation ahead, the column shared by two rotations stays in a
-//     register, and the negligible off-diagonal is found by all lanes;
+//     register, and the negligible off-diagonal is found by all lanes.  The
+//     lanes meet after every rotation;
 //   * Householder: p = tau A v by rows, the rank-2 update by columns, Q by
 //     columns; the reflector scalars are computed redundantly.
 // Shared arrays written by one lane and read by others are separated by
@@ -109,6 +110,10 @@ __device__ inline int tql_implicit(int n, double *d, double *e, double *Z, int l
                 d1 = di;
                 di = dn;
                 ei = en;
+                // Lane 0 writes entry i + 1 of d and e and the others read
+                // entry i - 1: a lane behind by two rotations would read a
+                // new value.
+                __syncwarp();
             }
 #pragma unroll
             for (int u = 0; u < RZ; ++u) {
