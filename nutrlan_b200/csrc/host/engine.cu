@@ -1284,12 +1284,15 @@ int Engine<T>::spec_segment(int *jnd_io, int S, int kept) {
     if constexpr (kWide) {
         if (coop_steps(j0)) {
             if (upload_run(j0, kept)) return -1001;
+            // TRLX_COOP_POLLS shortens the grid barrier's wait (to test what follows).
+            const char *e = std::getenv("TRLX_COOP_POLLS");
+            const long polls = e ? std::max(0L, std::min(kCoopPolls, std::strtol(e, nullptr, 10))) : kCoopPolls;
             int pid = pbeg();
             const int rc = launch_coop<C>(builtin_, reinterpret_cast<C *const *>(d_cols_),
                                           reinterpret_cast<C *>(col(maxlan_ + 1)),
                                           reinterpret_cast<C *>(col(maxlan_ + 2)), n_pad_, j0, S, kept, d_sc_ta_,
                                           d_sc_tb_, d_log_, d_sc_dot_, static_cast<double *>(scratch_.partials),
-                                          (size_t)scratch_.max_blocks * (P_ + 2) * 2, scratch_.tickets + 5, st_);
+                                          (size_t)scratch_.max_blocks * (P_ + 2) * 2, scratch_.tickets + 5, polls, st_);
             if (rc == -1001) return -1001;
             if (rc == 0) {
                 double bytes = 0.0;

@@ -47,7 +47,6 @@ namespace {
 // 16 warps on the rows of the product and two that form the pass's
 // coefficients and scalars meanwhile; all 18 in the other phases.
 constexpr int kThreads = 576;
-constexpr long kSpinLimit = 1L << 22;  // polls of the grid barrier before it gives up
 
 __device__ __forceinline__ double mulx(double a, double x) { return a * x; }
 __device__ __forceinline__ zd mulx(zd a, zd x) { return zd{a.x * x.x - a.y * x.y, a.x * x.y + a.y * x.x}; }
@@ -157,22 +156,22 @@ __device__ __forceinline__ double peer_double(const double *p, unsigned rank) {
 
 // Barrier over the grid (all blocks resident: a cooperative launch), after
 // the caller's cluster met: one block of a cluster arrives for all, every
-// block waits, for at most `limit` polls.  False when that ran out; the run
-// goes on without waiting then (its results are not used), so that the blocks
-// of a cluster keep meeting and end together.
-__device__ __forceinline__ bool grid_meet(unsigned *counter, unsigned target, bool arrive, long limit, int *flag) {
+// block waits, for at most `polls` looks.  *gave_up is set when that ran out;
+// the block goes on without waiting then (its results are not used) and keeps
+// meeting its cluster.  It no longer waits for the cluster's first block to
+// have read its sums, so it must neither write them again nor end before that.
+__device__ __forceinline__ void grid_meet(unsigned *counter, unsigned target, bool arrive, long polls, int *gave_up) {
     __syncthreads();
     if (threadIdx.x == 0) {
         if (arrive) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
-        long i = 0;
+        long i = *gave_up ? polls : 0;
         unsigned seen;
         do {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
-        } while (seen < target && ++i < limit);
-        *flag = seen < target;
+        } while (seen < target && ++i < polls);
+        if (seen < target) *gave_up = 1;
     }
     __syncthreads();
-    return *flag == 0;
 }
 
 // Sums of N values (a power of two) over the lanes of a warp, halving the
@@ -224,6 +223,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_coop(const CoopArgs<C> A) {
     const int rows = (int)max(0L, min((long)chunk, A.n_pad - r0));
 
     // ---- the block's state for the run -----------------------------------
+    if (tid == 0) gave_up = 0;
     for (int i = tid; i < A.j0; i += kThreads) {
         ta[i] = A.ta[i];
         tb[i] = A.tb[i];
@@ -282,7 +282,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_coop(const CoopArgs<C> A) {
     __syncthreads();
 
     double sigma = ta[A.j0 - 1], delta = 0.0;
-    bool ok = true;
     unsigned meets = 0;
     // Adds the clusters' partial sums of the step that made column k (into
     // tot), forms delta and the new sigma.
@@ -539,8 +538,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_coop(const CoopArgs<C> A) {
         }
         __syncthreads();
         // ---- partial p, g of every column (most warps); |z|^2, Re p_k, g_k ------
+        // (not over sums that the cluster's first block may still be reading)
         const int D = step_doubles<C>(k);
-        if (warp < W - 3) {
+        if (gave_up) {
+        } else if (warp < W - 3) {
             constexpr int NCW = 4 / cw;         // columns per warp and round
             constexpr int NV = 2 * cw * NCW;
             for (int c0 = warp * NCW; c0 <= k; c0 += (W - 3) * NCW) {
@@ -619,7 +620,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_coop(const CoopArgs<C> A) {
                 po[d + 1] = t.c;
             }
         }
-        ok = grid_meet(A.sync, ++meets * (unsigned)NCl, crank == 0, ok ? kSpinLimit : 0, &gave_up) && ok;
+        grid_meet(A.sync, ++meets * (unsigned)NCl, crank == 0, A.polls, &gave_up);
     }
     // ---- the last vector ------------------------------------------------------
     {
@@ -641,9 +642,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_coop(const CoopArgs<C> A) {
             out[r0 + i] = sc * ((sz[i] - delta * sv[i]) - u);
         }
     }
-    if (!ok && tid == 0) *A.failed = 1.0;  // the host takes no step of the run
+    if (gave_up && tid == 0) *A.failed = 1.0;  // the host takes no step of the run
+    cluster_meet();  // no block ends while its cluster's first may be reading its sums
     // The last block out leaves the counters at zero.
-    __syncthreads();
     if (tid == 0) {
         __threadfence();
         if (atomicAdd(A.sync + 1, 1u) == (unsigned)gridDim.x - 1) {
@@ -658,7 +659,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_coop(const CoopArgs<C> A) {
 template <class C>
 int launch_coop(const trlx_operator *A, C *const *cols, C *z0, C *z1, long n_pad, int j0, int S, int kept,
                 const double *ta, const double *tb, double *log, double *failed, double *part, size_t part_doubles,
-                unsigned *sync, cudaStream_t st) {
+                unsigned *sync, long polls, cudaStream_t st) {
     if (!A || S < 1 || j0 < 1 || op_complex(A) != (sizeof(C) == 16)) return -1;
     if (op_sell(A) && A->perm) return -1;
     // Per device, set up once: blocks of clusters of 8 and of 4 that are
@@ -739,6 +740,7 @@ int launch_coop(const trlx_operator *A, C *const *cols, C *z0, C *z1, long n_pad
     a.failed = failed;
     a.part = part;
     a.sync = sync;
+    a.polls = polls;
     const size_t smem = L.end + (size_t)a.nres * chunk * sizeof(C) + ecap * per;
     attr[0].val.clusterDim.x = cs;
     cfg.gridDim = dim3((unsigned)G);
@@ -748,8 +750,9 @@ int launch_coop(const trlx_operator *A, C *const *cols, C *z0, C *z1, long n_pad
 
 template int launch_coop<double>(const trlx_operator *, double *const *, double *, double *, long, int, int, int,
                                  const double *, const double *, double *, double *, double *, size_t, unsigned *,
-                                 cudaStream_t);
+                                 long, cudaStream_t);
 template int launch_coop<zd>(const trlx_operator *, zd *const *, zd *, zd *, long, int, int, int, const double *,
-                             const double *, double *, double *, double *, size_t, unsigned *, cudaStream_t);
+                             const double *, double *, double *, double *, size_t, unsigned *, long,
+                             cudaStream_t);
 
 }  // namespace trlb

@@ -31,7 +31,10 @@ struct CoopArgs {
     double *failed;  // set to 1 when a barrier gave up
     double *part;    // two sets of the clusters' partial sums
     unsigned *sync;  // two counters, zero between launches
+    long polls;      // of the grid barrier before it gives up
 };
+
+constexpr long kCoopPolls = 1L << 22;  // some seconds
 
 // Runs S steps of a built-in CSR operator or an unsorted SELL one.  Returns
 // 0, -1 if the kernel does not apply (operator form, device, sizes), -1001
@@ -39,6 +42,6 @@ struct CoopArgs {
 template <class C>
 int launch_coop(const trlx_operator *A, C *const *cols, C *z0, C *z1, long n_pad, int j0, int S, int kept,
                 const double *ta, const double *tb, double *log, double *failed, double *part, size_t part_doubles,
-                unsigned *sync, cudaStream_t st);
+                unsigned *sync, long polls, cudaStream_t st);
 
 }  // namespace trlb
