@@ -287,7 +287,7 @@ class Engine {
     static bool in_range(double beta) { return beta > 1e-90 && beta < 1e90; }
     bool sweeps(int jnd) const;
     bool coop_steps(int jnd) const;
-    int upload_run(int j0, int kept);
+    int upload_run(int j0, int S, int kept);
     int sweep_steps(int j0, int S, int kept);
     bool accept_step(int jnd, int kept, const double *lg, bool sweep);
     void track_ritz(int nd) {
@@ -359,7 +359,7 @@ class Engine {
     double *d_Y_ = nullptr;
     double *d_log_ = nullptr, *h_log_ = nullptr;  // speculative steps: alpha, |r|^2 pre/post, |h|^2
     // Single-sweep steps: V^H r (in d_coef_), T h, alphas, betas and scalars,
-    // contiguous, with the pinned copy a run starts from.
+    // contiguous and before the log, with the pinned copy a run starts from.
     C *d_sc_c_ = nullptr;
     double *d_sc_ta_ = nullptr, *d_sc_tb_ = nullptr, *d_sc_s_ = nullptr, *d_sc_dot_ = nullptr;
     double *h_sweep_ = nullptr;
@@ -541,7 +541,7 @@ int Engine<T>::setup() {
     d_scal_ = reinterpret_cast<double *>(sp + b_coef);
     d_Y_ = reinterpret_cast<double *>(sp + b_coef + b_scal);
     d_cols_ = reinterpret_cast<T **>(sp + b_coef + b_scal + b_Y);
-    const size_t host_len = 4 + log_len + sweep_doubles();
+    const size_t host_len = 4 + log_len + sweep_doubles() + log_len;
     if (ws.h_log_len < host_len) {
         cudaFreeHost(ws.h_log);
         ws.h_log = nullptr;
@@ -1190,12 +1190,16 @@ bool Engine<T>::accept_step(int jnd, int kept, const double *lg, bool sweep) {
     return true;
 }
 
-// What a run of single-sweep steps from basis size j0 starts from: T, and
-// the first product's coefficients (it is of a finished vector: nothing to
-// correct, scale 1).
+// What a run of S single-sweep steps from basis size j0 starts from: T, the
+// first product's coefficients (it is of a finished vector: nothing to
+// correct, scale 1), and a log without numbers, which accept_step takes no
+// step from: an entry that no kernel writes is not read as one of an earlier
+// run.
 template <class T>
-int Engine<T>::upload_run(int j0, int kept) {
+int Engine<T>::upload_run(int j0, int S, int kept) {
     std::memset(h_sweep_, 0, sizeof(double) * sweep_doubles());
+    const size_t log = 4 * ((size_t)S + 1);
+    std::fill_n(h_sweep_ + sweep_doubles(), log, std::nan(""));
     double *hc = h_sweep_ + (sizeof(C) / sizeof(double)) * (size_t)P_;
     double *hta = hc + (sizeof(C) / sizeof(double)) * (size_t)P_, *htb = hta + P_, *hs = htb + P_;
     // The step after a restart (j0 == kept) has the arrowhead row for its
@@ -1212,7 +1216,7 @@ int Engine<T>::upload_run(int j0, int kept) {
     }
     hs[0] = hs[1] = 1.0;
     hs[2] = j0 == kept ? 0.0 : beta_[j0 - 1];
-    CK(cudaMemcpyAsync(d_coef_, h_sweep_, sizeof(double) * sweep_doubles(), cudaMemcpyHostToDevice, st_));
+    CK(cudaMemcpyAsync(d_coef_, h_sweep_, sizeof(double) * (sweep_doubles() + log), cudaMemcpyHostToDevice, st_));
     return 0;
 }
 
@@ -1222,7 +1226,7 @@ int Engine<T>::upload_run(int j0, int kept) {
 // normalisation.  The steps log what the discrete kernels log.
 template <class T>
 int Engine<T>::sweep_steps(int j0, int S, int kept) {
-    if (int e = upload_run(j0, kept)) return e;
+    if (int e = upload_run(j0, S, kept)) return e;
     for (int s = 1; s <= S; ++s) {
         const int k = j0 + s - 1;
         SweepArgs<T> w;
@@ -1255,7 +1259,7 @@ int Engine<T>::sweep_steps(int j0, int S, int kept) {
         w.lg = d_log_ + 4 * (size_t)s;
         w.lg_prev = w.lg - 4;
         pid = pbeg();
-        launch_sweep<T>(w, scratch_, st_);
+        if (int e = launch_sweep<T>(w, scratch_, st_)) return e;
         pend(pid, TRLX_K_PROJECT,
              (double)nrow_ * (k * sv() + (s == 1 ? 3.0 : 4.0) * cs() + (kWide ? 0.0 : cs() + sv())));
         rotate_fp64();
@@ -1283,7 +1287,7 @@ int Engine<T>::spec_segment(int *jnd_io, int S, int kept) {
     // Short vectors: the whole run in one cooperative kernel.
     if constexpr (kWide) {
         if (coop_steps(j0)) {
-            if (upload_run(j0, kept)) return -1001;
+            if (upload_run(j0, S, kept)) return -1001;
             // TRLX_COOP_POLLS shortens the grid barrier's wait (to test what follows).
             const char *e = std::getenv("TRLX_COOP_POLLS");
             const long polls = e ? std::max(0L, std::min(kCoopPolls, std::strtol(e, nullptr, 10))) : kCoopPolls;

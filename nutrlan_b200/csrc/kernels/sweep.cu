@@ -471,7 +471,7 @@ constexpr Variant<T> variant() {
 }  // namespace
 
 template <class T>
-void launch_sweep(const SweepArgs<T> &a, Scratch &s, cudaStream_t st) {
+int launch_sweep(const SweepArgs<T> &a, Scratch &s, cudaStream_t st) {
     using C = typename Store<T>::C;
     // By groups (1, 2, 4, 8) and columns per group (to 8 or 10, 12, 14, 16).
     static const Variant<T> kern[4][4] = {
@@ -489,7 +489,9 @@ void launch_sweep(const SweepArgs<T> &a, Scratch &s, cudaStream_t st) {
         if (sms <= 0) sms = 148;
         for (const auto &row : kern)
             for (const auto &v : row)
-                cudaFuncSetAttribute(v.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem);
+                if (cudaFuncSetAttribute(v.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem) !=
+                    cudaSuccess)
+                    return -1001;
         if (dev < 64) sms_of[dev] = sms;
     }
     // One block per SM on an equal share of the rows, in whole tiles.
@@ -518,12 +520,13 @@ void launch_sweep(const SweepArgs<T> &a, Scratch &s, cudaStream_t st) {
     cfg.stream = st;
     cfg.attrs = &early;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, v.kern, a, chunk, part, part_r2, s.tickets + kTicketSweep);
+    return cudaLaunchKernelEx(&cfg, v.kern, a, chunk, part, part_r2, s.tickets + kTicketSweep) == cudaSuccess ? 0
+                                                                                                            : -1001;
 }
 
-template void launch_sweep<double>(const SweepArgs<double> &, Scratch &, cudaStream_t);
-template void launch_sweep<float>(const SweepArgs<float> &, Scratch &, cudaStream_t);
-template void launch_sweep<zd>(const SweepArgs<zd> &, Scratch &, cudaStream_t);
-template void launch_sweep<zf>(const SweepArgs<zf> &, Scratch &, cudaStream_t);
+template int launch_sweep<double>(const SweepArgs<double> &, Scratch &, cudaStream_t);
+template int launch_sweep<float>(const SweepArgs<float> &, Scratch &, cudaStream_t);
+template int launch_sweep<zd>(const SweepArgs<zd> &, Scratch &, cudaStream_t);
+template int launch_sweep<zf>(const SweepArgs<zf> &, Scratch &, cudaStream_t);
 
 }  // namespace trlb

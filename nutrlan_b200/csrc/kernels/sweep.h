@@ -34,7 +34,8 @@ struct SweepArgs {
     double *lg_prev = nullptr;  // log of step k (its last entry is written here)
 };
 
+// 0, or -1001 if the kernel was not launched.
 template <class T>
-void launch_sweep(const SweepArgs<T> &a, Scratch &s, cudaStream_t st);
+int launch_sweep(const SweepArgs<T> &a, Scratch &s, cudaStream_t st);
 
 }  // namespace trlb
