@@ -279,11 +279,13 @@ class Engine {
     int read_checkpoint(int nec, int *jnd_out);
     int refine_fp64(int k, double *max_res);
     bool spec_enabled() const;
+    // The steps accepted (jnd moves on by them), or an error.
     int spec_segment(int *jnd, int S, int kept);
     // Asked of every beta of a run of single-sweep steps: keeps |r|^2 and
     // r^H A r, formed from unnormalised vectors, far from overflow and
     // underflow.  A solve that meets another goes on without such runs.
     bool scale_off_ = false;
+    bool sweep_off_ = false;  // a sweep's launch or memory was refused: the solve goes on without
     static bool in_range(double beta) { return beta > 1e-90 && beta < 1e90; }
     bool sweeps(int jnd) const;
     bool coop_steps(int jnd) const;
@@ -1128,7 +1130,8 @@ bool Engine<T>::spec_enabled() const {
 template <class T>
 bool Engine<T>::sweeps(int jnd) const {
     // A 32-bit basis has no other speculative steps, so any length counts.
-    if ((kWide && n_pad_ < kSweepMinRows) || jnd < 1 || jnd + 1 > kSweepCols || scale_off_) return false;
+    if ((kWide && n_pad_ < kSweepMinRows) || jnd < 1 || jnd + 1 > kSweepCols || scale_off_ || sweep_off_)
+        return false;
     if ((size_t)P_ * n_pad_ * sizeof(T) > (1ull << 36)) return false;  // 32-bit column offsets, 16-byte units
     const char *e = std::getenv("TRLX_SWEEP");
     return !(e && e[0] == '0');
@@ -1297,7 +1300,6 @@ int Engine<T>::spec_segment(int *jnd_io, int S, int kept) {
                                           reinterpret_cast<C *>(col(maxlan_ + 2)), n_pad_, j0, S, kept, d_sc_ta_,
                                           d_sc_tb_, d_log_, d_sc_dot_, static_cast<double *>(scratch_.partials),
                                           (size_t)scratch_.max_blocks * (P_ + 2) * 2, scratch_.tickets + 5, polls, st_);
-            if (rc == -1001) return -1001;
             if (rc == 0) {
                 double bytes = 0.0;
                 for (int s = 1; s <= S; ++s) bytes += spmv_bytes(builtin_) + ((double)(j0 + s) + 4.0) * nrow_ * cs();
@@ -1309,18 +1311,35 @@ int Engine<T>::spec_segment(int *jnd_io, int S, int kept) {
             }
         }
     }
+    // The FP64 working vectors of a 32-bit basis at the run's start, which a
+    // rejected step or a run that was not issued goes back to.
+    const size_t vec = sizeof(C) * n_pad_;
+    auto go_back = [&]() -> int {
+        Workspace &ws = workspace();
+        CK(cudaMemcpyAsync(qa64_, ws.saved, vec, cudaMemcpyDeviceToDevice, st_));
+        CK(cudaMemcpyAsync(qb64_, static_cast<char *>(ws.saved) + vec, vec, cudaMemcpyDeviceToDevice, st_));
+        return 0;
+    };
     if (!done && sweeps(j0)) {
         if constexpr (!kWide) {
-            // The FP64 working vectors a rejected step goes back to.
             Workspace &ws = workspace();
-            const size_t vec = sizeof(C) * n_pad_;
-            if (!Workspace::ensure(&ws.saved, &ws.saved_bytes, 2 * vec)) return 0;
+            if (!Workspace::ensure(&ws.saved, &ws.saved_bytes, 2 * vec)) {
+                sweep_off_ = true;  // no memory for them: steps one by one
+                return 0;
+            }
             CK(cudaMemcpyAsync(ws.saved, qa64_, vec, cudaMemcpyDeviceToDevice, st_));
             CK(cudaMemcpyAsync(static_cast<char *>(ws.saved) + vec, qb64_, vec, cudaMemcpyDeviceToDevice, st_));
         }
-        if (sweep_steps(j0, S, kept)) return -1001;
-        info_->matvec += S;
-        done = sweep = true;
+        const int rc = sweep_steps(j0, S, kept);
+        if (rc == -1001) return rc;
+        if (rc == 0) {
+            info_->matvec += S;
+            done = sweep = true;
+        } else {
+            sweep_off_ = true;
+            if constexpr (!kWide)
+                if (int e = go_back()) return e;
+        }
     }
     if constexpr (kWide) {
         for (int s = 1; s <= S && !done; ++s) {
@@ -1379,10 +1398,7 @@ int Engine<T>::spec_segment(int *jnd_io, int S, int kept) {
         if (dropped) {
             // The working vectors moved on: back to the run's start, and the
             // accepted steps again (the same kernels on the same values).
-            Workspace &ws = workspace();
-            const size_t vec = sizeof(C) * n_pad_;
-            CK(cudaMemcpyAsync(qa64_, ws.saved, vec, cudaMemcpyDeviceToDevice, st_));
-            CK(cudaMemcpyAsync(qb64_, static_cast<char *>(ws.saved) + vec, vec, cudaMemcpyDeviceToDevice, st_));
+            if (int e = go_back()) return e;
             if (acc > 0 && sweep_steps(j0, acc, kept)) return -1001;
             discarded_ += acc;
             CK(cudaStreamSynchronize(st_));
@@ -1655,7 +1671,11 @@ void Engine<T>::run() {
             // the first step.
             run = std::min<long>((long)info->klan - jnd, std::max<long>(2, (long)next_test - info->matvec));
             if (sweeps(jnd)) run = std::min<long>(run, kSweepCols + 1 - jnd);
-            if (run >= 2) acc = std::max(spec_segment(&jnd, (int)run, kept), 0);
+            if (run >= 2) acc = spec_segment(&jnd, (int)run, kept);
+            if (acc < 0) {
+                stat = acc;
+                break;
+            }
         }
         if (acc == 0) {
         // ---- first step after (re)start: arrowhead coupling -------------------
@@ -1746,6 +1766,10 @@ void Engine<T>::run() {
                 else S = 1;
                 if (S >= 2 || (S == 1 && coop_steps(jnd))) {
                     const int acc = spec_segment(&jnd, (int)S, kept);
+                    if (acc < 0) {
+                        stat = acc;
+                        break;
+                    }
                     if (acc == S) {
                         if (info->matvec >= next_test && (stat = test_convergence())) break;
                         continue;

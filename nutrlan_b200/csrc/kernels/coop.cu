@@ -745,7 +745,9 @@ int launch_coop(const trlx_operator *A, C *const *cols, C *z0, C *z1, long n_pad
     attr[0].val.clusterDim.x = cs;
     cfg.gridDim = dim3((unsigned)G);
     cfg.dynamicSmemBytes = smem;
-    return cudaLaunchKernelEx(&cfg, k_coop<C>, a) == cudaSuccess ? 0 : -1001;
+    if (cudaLaunchKernelEx(&cfg, k_coop<C>, a) == cudaSuccess) return 0;
+    cudaGetLastError();
+    return -1;
 }
 
 template int launch_coop<double>(const trlx_operator *, double *const *, double *, double *, long, int, int, int,

@@ -37,8 +37,8 @@ struct CoopArgs {
 constexpr long kCoopPolls = 1L << 22;  // some seconds
 
 // Runs S steps of a built-in CSR operator or an unsorted SELL one.  Returns
-// 0, -1 if the kernel does not apply (operator form, device, sizes), -1001
-// on a CUDA error.
+// 0, or -1 if the kernel does not apply (operator form, device, sizes) or was
+// not launched (nothing is changed then).
 template <class C>
 int launch_coop(const trlx_operator *A, C *const *cols, C *z0, C *z1, long n_pad, int j0, int S, int kept,
                 const double *ta, const double *tb, double *log, double *failed, double *part, size_t part_doubles,

@@ -490,8 +490,10 @@ int launch_sweep(const SweepArgs<T> &a, Scratch &s, cudaStream_t st) {
         for (const auto &row : kern)
             for (const auto &v : row)
                 if (cudaFuncSetAttribute(v.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem) !=
-                    cudaSuccess)
-                    return -1001;
+                    cudaSuccess) {
+                    cudaGetLastError();
+                    return -1;
+                }
         if (dev < 64) sms_of[dev] = sms;
     }
     // One block per SM on an equal share of the rows, in whole tiles.
@@ -520,8 +522,9 @@ int launch_sweep(const SweepArgs<T> &a, Scratch &s, cudaStream_t st) {
     cfg.stream = st;
     cfg.attrs = &early;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, v.kern, a, chunk, part, part_r2, s.tickets + kTicketSweep) == cudaSuccess ? 0
-                                                                                                            : -1001;
+    if (cudaLaunchKernelEx(&cfg, v.kern, a, chunk, part, part_r2, s.tickets + kTicketSweep) == cudaSuccess) return 0;
+    cudaGetLastError();
+    return -1;
 }
 
 template int launch_sweep<double>(const SweepArgs<double> &, Scratch &, cudaStream_t);

@@ -34,7 +34,7 @@ struct SweepArgs {
     double *lg_prev = nullptr;  // log of step k (its last entry is written here)
 };
 
-// 0, or -1001 if the kernel was not launched.
+// 0, or -1 if the kernel was not launched (nothing is changed then).
 template <class T>
 int launch_sweep(const SweepArgs<T> &a, Scratch &s, cudaStream_t st);
 
