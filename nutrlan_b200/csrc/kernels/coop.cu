@@ -36,6 +36,7 @@
 // each) and two passes over the chunk in shared memory.
 #include <algorithm>
 #include <cstdlib>
+#include <mutex>
 
 #include "coop.h"
 #include "spmv.h"
@@ -663,8 +664,11 @@ int launch_coop(const trlx_operator *A, C *const *cols, C *z0, C *z1, long n_pad
     if (!A || S < 1 || j0 < 1 || op_complex(A) != (sizeof(C) == 16)) return -1;
     if (op_sell(A) && A->perm) return -1;
     // Per device, set up once: blocks of clusters of 8 and of 4 that are
-    // resident together, one per SM (-1: no cooperative launch).
+    // resident together, one per SM (-1: no cooperative launch).  Host threads
+    // take turns: none sees a device half set up.
+    static std::mutex turn;
     static int blocks_of[64][2] = {};
+    int blocks[2];
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return -1;
@@ -679,28 +683,33 @@ int launch_coop(const trlx_operator *A, C *const *cols, C *z0, C *z1, long n_pad
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    if (blocks_of[dev][0] == 0) {
-        int coop = 0;
-        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-        if (cudaFuncSetAttribute(k_coop<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess)
-            coop = 0;
-        for (int i = 0; i < 2; ++i) {
-            const int cs = i == 0 ? 8 : 4;
-            attr[0].val.clusterDim.x = cs;
-            cfg.gridDim = dim3(cs);
-            cfg.dynamicSmemBytes = kMaxSmem;
-            int n = 0;
-            if (!coop || cudaOccupancyMaxActiveClusters(&n, k_coop<C>, &cfg) != cudaSuccess) n = 0;
-            blocks_of[dev][i] = n > 0 ? n * cs : -1;
+    {
+        std::lock_guard<std::mutex> hold(turn);
+        if (blocks_of[dev][0] == 0) {
+            int coop = 0;
+            cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+            if (cudaFuncSetAttribute(k_coop<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess)
+                coop = 0;
+            for (int i = 0; i < 2; ++i) {
+                const int cs = i == 0 ? 8 : 4;
+                attr[0].val.clusterDim.x = cs;
+                cfg.gridDim = dim3(cs);
+                cfg.dynamicSmemBytes = kMaxSmem;
+                int n = 0;
+                if (!coop || cudaOccupancyMaxActiveClusters(&n, k_coop<C>, &cfg) != cudaSuccess) n = 0;
+                blocks_of[dev][i] = n > 0 ? n * cs : -1;
+            }
+            cudaGetLastError();
         }
-        cudaGetLastError();
+        blocks[0] = blocks_of[dev][0];
+        blocks[1] = blocks_of[dev][1];
     }
     // Clusters of 8 while their blocks keep 256 rows or fewer; of 4, which
     // cover more SMs, for longer vectors.
-    int cs = 8, most = blocks_of[dev][0];
+    int cs = 8, most = blocks[0];
     if (most < 0 || n_pad > 256L * most) {
         cs = 4;
-        most = blocks_of[dev][1];
+        most = blocks[1];
     }
     if (most < cs) return -1;
     const long chunk = ((n_pad + most - 1) / most + 31) / 32 * 32;

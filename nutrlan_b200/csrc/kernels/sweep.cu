@@ -30,6 +30,7 @@
 // FP64 copy, V T h is formed from the stored columns (h is then of the size
 // of the storage rounding, and its error of that size squared).
 #include <algorithm>
+#include <mutex>
 #include <type_traits>
 
 #include "sweep.h"
@@ -479,22 +480,27 @@ int launch_sweep(const SweepArgs<T> &a, Scratch &s, cudaStream_t st) {
         {variant<T, 10, 2>(), variant<T, 12, 2>(), variant<T, 14, 2>(), variant<T, 16, 2>()},
         {variant<T, 10, 4>(), variant<T, 12, 4>(), variant<T, 14, 4>(), variant<T, 16, 4>()},
         {variant<T, 10, 8>(), variant<T, 12, 8>(), variant<T, 14, 8>(), variant<T, 16, 8>()}};
-    // SMs of each device; reading them also lets the kernels use their ring there.
+    // SMs of each device; reading them also lets the kernels use their ring
+    // there.  Host threads take turns: none sees a device half set up.
+    static std::mutex turn;
     static int sms_of[64] = {};
-    int dev = 0;
+    int dev = 0, sms = 0;
     cudaGetDevice(&dev);
-    int sms = dev < 64 ? sms_of[dev] : 0;
-    if (sms == 0) {
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 148;
-        for (const auto &row : kern)
-            for (const auto &v : row)
-                if (cudaFuncSetAttribute(v.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem) !=
-                    cudaSuccess) {
-                    cudaGetLastError();
-                    return -1;
-                }
-        if (dev < 64) sms_of[dev] = sms;
+    {
+        std::lock_guard<std::mutex> hold(turn);
+        if (dev < 64) sms = sms_of[dev];
+        if (sms == 0) {
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            if (sms <= 0) sms = 148;
+            for (const auto &row : kern)
+                for (const auto &v : row)
+                    if (cudaFuncSetAttribute(v.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem) !=
+                        cudaSuccess) {
+                        cudaGetLastError();
+                        return -1;
+                    }
+            if (dev < 64) sms_of[dev] = sms;
+        }
     }
     // One block per SM on an equal share of the rows, in whole tiles.
     const long tile = 32 * Store<T>::R;

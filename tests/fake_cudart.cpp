@@ -11,6 +11,8 @@ int fake_device, fake_attribute_answer;
 int fake_launch_answer;   // of cudaLaunchKernelEx (sweeps and cooperative runs)
 int fake_launches;        // how many of those were asked for
 int fake_sync_failures;   // so many waits fail after the first of those launches
+void (*fake_on_occupancy)(int call);  // called by the occupancy query of clusters, with its number
+int fake_occupancy_calls;
 
 static void *ones(size_t bytes) {
     double *p = (double *)malloc(bytes + 256);
@@ -33,6 +35,8 @@ cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr a, int) {
 cudaError_t cudaFuncSetAttribute(const void *, cudaFuncAttribute, int) { return (cudaError_t)fake_attribute_answer; }
 cudaError_t cudaOccupancyMaxActiveClusters(int *n, const void *, const cudaLaunchConfig_t *) {
     *n = 16;
+    const int call = ++fake_occupancy_calls;
+    if (fake_on_occupancy) fake_on_occupancy(call);
     return cudaSuccess;
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const void *, int, size_t, unsigned) {
