@@ -286,9 +286,11 @@ class Engine {
     // underflow.  A solve that meets another goes on without such runs.
     bool scale_off_ = false;
     bool sweep_off_ = false;  // a sweep's launch or memory was refused: the solve goes on without
+    bool coop_off_ = false;   // the same of a cooperative run's launch
     static bool in_range(double beta) { return beta > 1e-90 && beta < 1e90; }
     bool sweeps(int jnd) const;
-    bool coop_steps(int jnd) const;
+    bool coop_steps(int jnd, int S) const;
+    size_t partial_doubles() const { return (size_t)scratch_.max_blocks * (P_ + 2) * 2; }
     int upload_run(int j0, int S, int kept);
     int sweep_steps(int j0, int S, int kept);
     bool accept_step(int jnd, int kept, const double *lg, bool sweep);
@@ -1137,12 +1139,15 @@ bool Engine<T>::sweeps(int jnd) const {
     return !(e && e[0] == '0');
 }
 
-// Whether they run in the cooperative kernel (coop.h).
+// Whether S of them run in the cooperative kernel (coop.h).
 template <class T>
-bool Engine<T>::coop_steps(int jnd) const {
-    if (!kWide || jnd < 1 || n_pad_ >= kSweepMinRows || scale_off_) return false;
-    const char *e = std::getenv("TRLX_COOP");
-    return !(e && e[0] == '0');
+bool Engine<T>::coop_steps(int jnd, int S) const {
+    if constexpr (kWide) {
+        if (jnd < 1 || n_pad_ >= kSweepMinRows || scale_off_ || coop_off_) return false;
+        const char *e = std::getenv("TRLX_COOP");
+        return !(e && e[0] == '0') && coop_applies<C>(builtin_, n_pad_, jnd + S, partial_doubles());
+    }
+    return false;
 }
 
 template <class T>
@@ -1289,7 +1294,7 @@ int Engine<T>::spec_segment(int *jnd_io, int S, int kept) {
     bool done = false, sweep = false, coop = false;
     // Short vectors: the whole run in one cooperative kernel.
     if constexpr (kWide) {
-        if (coop_steps(j0)) {
+        if (coop_steps(j0, S)) {
             if (upload_run(j0, S, kept)) return -1001;
             // TRLX_COOP_POLLS shortens the grid barrier's wait (to test what follows).
             const char *e = std::getenv("TRLX_COOP_POLLS");
@@ -1299,7 +1304,7 @@ int Engine<T>::spec_segment(int *jnd_io, int S, int kept) {
                                           reinterpret_cast<C *>(col(maxlan_ + 1)),
                                           reinterpret_cast<C *>(col(maxlan_ + 2)), n_pad_, j0, S, kept, d_sc_ta_,
                                           d_sc_tb_, d_log_, d_sc_dot_, static_cast<double *>(scratch_.partials),
-                                          (size_t)scratch_.max_blocks * (P_ + 2) * 2, scratch_.tickets + 5, polls, st_);
+                                          partial_doubles(), scratch_.tickets + 5, polls, st_);
             if (rc == 0) {
                 double bytes = 0.0;
                 for (int s = 1; s <= S; ++s) bytes += spmv_bytes(builtin_) + ((double)(j0 + s) + 4.0) * nrow_ * cs();
@@ -1308,6 +1313,8 @@ int Engine<T>::spec_segment(int *jnd_io, int S, int kept) {
                 count_launch();
                 coop_segments_++;
                 done = coop = true;
+            } else {
+                coop_off_ = true;
             }
         }
     }
@@ -1341,6 +1348,9 @@ int Engine<T>::spec_segment(int *jnd_io, int S, int kept) {
                 if (int e = go_back()) return e;
         }
     }
+    // The discrete steps know the three-term recurrence only, not the
+    // arrowhead row of the step after a restart.
+    if (!done && j0 == kept) return 0;
     if constexpr (kWide) {
         for (int s = 1; s <= S && !done; ++s) {
             const int j = j0 + s;
@@ -1666,12 +1676,13 @@ void Engine<T>::run() {
         // ---- steps from the (re)start on, the arrowhead one first -------------
         int acc = 0;
         long run = 0;
-        if (spec_enabled() && (sweeps(jnd) || coop_steps(jnd))) {
+        if (spec_enabled()) {
             // Up to the next convergence test, which never comes right after
             // the first step.
             run = std::min<long>((long)info->klan - jnd, std::max<long>(2, (long)next_test - info->matvec));
-            if (sweeps(jnd)) run = std::min<long>(run, kSweepCols + 1 - jnd);
-            if (run >= 2) acc = spec_segment(&jnd, (int)run, kept);
+            const bool sweep = sweeps(jnd);
+            if (sweep) run = std::min<long>(run, kSweepCols + 1 - jnd);
+            if (run >= 2 && (sweep || coop_steps(jnd, (int)run))) acc = spec_segment(&jnd, (int)run, kept);
             if (acc < 0) {
                 stat = acc;
                 break;
@@ -1758,13 +1769,16 @@ void Engine<T>::run() {
         };
         if (acc > 1 && acc == run && info->matvec >= next_test && (stat = test_convergence())) break;
         while (jnd < info->klan && info->nec < info->ned) {
-            if (spec_enabled() && (kWide ? jnd >= 2 || sweeps(jnd) || coop_steps(jnd) : sweeps(jnd))) {
+            if (spec_enabled()) {
                 // Steps up to the next convergence test (or the restart).
                 long S = (long)info->klan - jnd;
-                if (sweeps(jnd)) S = std::min<long>(S, kSweepCols + 1 - jnd);
+                const bool sweep = sweeps(jnd);
+                if (sweep) S = std::min<long>(S, kSweepCols + 1 - jnd);
                 if (next_test > info->matvec) S = std::min<long>(S, (long)next_test - info->matvec);
                 else S = 1;
-                if (S >= 2 || (S == 1 && coop_steps(jnd))) {
+                // A single step pays as a cooperative run only, the discrete
+                // kernels need a column before the last.
+                if (S >= 2 ? sweep || (kWide && jnd >= 2) || coop_steps(jnd, (int)S) : coop_steps(jnd, (int)S)) {
                     const int acc = spec_segment(&jnd, (int)S, kept);
                     if (acc < 0) {
                         stat = acc;

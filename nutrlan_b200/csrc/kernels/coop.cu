@@ -655,14 +655,26 @@ __global__ void __launch_bounds__(kThreads, 1) k_coop(const CoopArgs<C> A) {
     }
 }
 
-}  // namespace
+constexpr size_t kMaxSmem = 220 * 1024;
 
+// How a run over `n_pad` rows and up to `kmax` columns is split.
+struct Plan {
+    int cluster, chunk, grid, nres, ecap;
+    size_t smem;
+};
+
+void set_cluster(cudaLaunchAttribute (&attr)[2], int blocks) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = blocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeCooperative;
+    attr[1].val.cooperative = 1;
+}
+
+// False where the kernel does not apply: operator form, device, sizes.
 template <class C>
-int launch_coop(const trlx_operator *A, C *const *cols, C *z0, C *z1, long n_pad, int j0, int S, int kept,
-                const double *ta, const double *tb, double *log, double *failed, double *part, size_t part_doubles,
-                unsigned *sync, long polls, cudaStream_t st) {
-    if (!A || S < 1 || j0 < 1 || op_complex(A) != (sizeof(C) == 16)) return -1;
-    if (op_sell(A) && A->perm) return -1;
+bool make_plan(const trlx_operator *A, long n_pad, int kmax, size_t part_doubles, Plan *p) {
+    if (!A || op_complex(A) != (sizeof(C) == 16) || (op_sell(A) && A->perm)) return false;
     // Per device, set up once: blocks of clusters of 8 and of 4 that are
     // resident together, one per SM (-1: no cooperative launch).  Host threads
     // take turns: none sees a device half set up.
@@ -671,30 +683,25 @@ int launch_coop(const trlx_operator *A, C *const *cols, C *z0, C *z1, long n_pad
     int blocks[2];
     int dev = 0;
     cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return -1;
-    constexpr int kMaxSmem = 220 * 1024;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeCooperative;
-    attr[1].val.cooperative = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(kThreads);
-    cfg.stream = st;
-    cfg.attrs = attr;
-    cfg.numAttrs = 2;
+    if (dev < 0 || dev >= 64) return false;
     {
         std::lock_guard<std::mutex> hold(turn);
         if (blocks_of[dev][0] == 0) {
             int coop = 0;
             cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-            if (cudaFuncSetAttribute(k_coop<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess)
+            if (cudaFuncSetAttribute(k_coop<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem) !=
+                cudaSuccess)
                 coop = 0;
+            cudaLaunchAttribute attr[2];
+            cudaLaunchConfig_t cfg = {};
+            cfg.blockDim = dim3(kThreads);
+            cfg.dynamicSmemBytes = kMaxSmem;
+            cfg.attrs = attr;
+            cfg.numAttrs = 2;
             for (int i = 0; i < 2; ++i) {
                 const int cs = i == 0 ? 8 : 4;
-                attr[0].val.clusterDim.x = cs;
+                set_cluster(attr, cs);
                 cfg.gridDim = dim3(cs);
-                cfg.dynamicSmemBytes = kMaxSmem;
                 int n = 0;
                 if (!coop || cudaOccupancyMaxActiveClusters(&n, k_coop<C>, &cfg) != cudaSuccess) n = 0;
                 blocks_of[dev][i] = n > 0 ? n * cs : -1;
@@ -711,24 +718,46 @@ int launch_coop(const trlx_operator *A, C *const *cols, C *z0, C *z1, long n_pad
         cs = 4;
         most = blocks[1];
     }
-    if (most < cs) return -1;
+    if (most < cs) return false;
     const long chunk = ((n_pad + most - 1) / most + 31) / 32 * 32;
-    const int G = (int)(((n_pad + chunk - 1) / chunk + cs - 1) / cs * cs);
-    CoopArgs<C> a;
-    a.kmax = j0 + S;
-    const Layout<C> L((int)chunk, a.kmax);
-    if (L.end > (size_t)kMaxSmem) return -1;
-    if ((size_t)2 * (G / cs) * step_doubles<C>(a.kmax) > part_doubles) return -1;
+    p->cluster = cs;
+    p->chunk = (int)chunk;
+    p->grid = (int)(((n_pad + chunk - 1) / chunk + cs - 1) / cs * cs);
+    const Layout<C> L((int)chunk, kmax);
+    if (L.end > kMaxSmem) return false;
+    if ((size_t)2 * (p->grid / cs) * step_doubles<C>(kmax) > part_doubles) return false;
     // Entries of a block in shared memory up to a third of what is left
     // (twice the average, for uneven rows), basis columns in the rest.
     const size_t left = kMaxSmem - L.end;
     const size_t per = sizeof(C) + sizeof(int);
-    size_t ecap = std::min<size_t>(left / 3 / per, (size_t)(2 * (A->nnz / G + 1) + 64)) / 4 * 4;
-    a.nres = (int)std::min<size_t>((left - ecap * per) / (sizeof(C) * chunk), (size_t)a.kmax);
-    a.ecap = (int)ecap;
+    const size_t ecap = std::min<size_t>(left / 3 / per, (size_t)(2 * (A->nnz / p->grid + 1) + 64)) / 4 * 4;
+    p->nres = (int)std::min<size_t>((left - ecap * per) / (sizeof(C) * chunk), (size_t)kmax);
+    p->ecap = (int)ecap;
+    p->smem = L.end + (size_t)p->nres * chunk * sizeof(C) + ecap * per;
+    return true;
+}
+
+}  // namespace
+
+template <class C>
+bool coop_applies(const trlx_operator *A, long n_pad, int kmax, size_t part_doubles) {
+    Plan p;
+    return make_plan<C>(A, n_pad, kmax, part_doubles, &p);
+}
+
+template <class C>
+int launch_coop(const trlx_operator *A, C *const *cols, C *z0, C *z1, long n_pad, int j0, int S, int kept,
+                const double *ta, const double *tb, double *log, double *failed, double *part, size_t part_doubles,
+                unsigned *sync, long polls, cudaStream_t st) {
+    Plan p;
+    if (S < 1 || j0 < 1 || !make_plan<C>(A, n_pad, j0 + S, part_doubles, &p)) return -1;
+    CoopArgs<C> a;
+    a.kmax = j0 + S;
+    a.nres = p.nres;
+    a.ecap = p.ecap;
     a.nrow = A->nrow;
     a.n_pad = n_pad;
-    a.chunk = (int)chunk;
+    a.chunk = p.chunk;
     // Lanes per row: one while a row's entries are loaded together anyway
     // (neighbouring rows of a lattice then read neighbouring values).
     a.tpr = 1;
@@ -750,15 +779,22 @@ int launch_coop(const trlx_operator *A, C *const *cols, C *z0, C *z1, long n_pad
     a.part = part;
     a.sync = sync;
     a.polls = polls;
-    const size_t smem = L.end + (size_t)a.nres * chunk * sizeof(C) + ecap * per;
-    attr[0].val.clusterDim.x = cs;
-    cfg.gridDim = dim3((unsigned)G);
-    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[2];
+    set_cluster(attr, p.cluster);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)p.grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = p.smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
     if (cudaLaunchKernelEx(&cfg, k_coop<C>, a) == cudaSuccess) return 0;
     cudaGetLastError();
     return -1;
 }
 
+template bool coop_applies<double>(const trlx_operator *, long, int, size_t);
+template bool coop_applies<zd>(const trlx_operator *, long, int, size_t);
 template int launch_coop<double>(const trlx_operator *, double *const *, double *, double *, long, int, int, int,
                                  const double *, const double *, double *, double *, double *, size_t, unsigned *,
                                  long, cudaStream_t);

@@ -36,6 +36,12 @@ struct CoopArgs {
 
 constexpr long kCoopPolls = 1L << 22;  // some seconds
 
+// Whether the kernel takes runs of this operator, up to `kmax` columns, on the
+// current device: CSR or unsorted SELL, sizes that fit in shared memory,
+// cooperative launches.
+template <class C>
+bool coop_applies(const trlx_operator *A, long n_pad, int kmax, size_t part_doubles);
+
 // Runs S steps of a built-in CSR operator or an unsorted SELL one.  Returns
 // 0, or -1 if the kernel does not apply (operator form, device, sizes) or was
 // not launched (nothing is changed then).

@@ -42,3 +42,40 @@ def test_cooperative_run_whose_barrier_gives_up_is_not_used(A, maxlan, maxmv, po
     assert full.stats.speculative_discarded == 0 and full.stats.speculative_steps > 0
     _same(cut, seq, 4)
     _same(full, seq, 4)
+
+
+def _uneven(n, cplx):
+    """A grid Laplacian with every eleventh row coupled to 12 more, so that a
+    SELL operator of sorted rows keeps them in another order."""
+    import scipy.sparse as sp
+    L = int(n ** 0.5)
+    A = ops.laplacian_2d(L, diag=2.0 * ops.uniform01(3, np.arange(L * L, dtype=np.uint64))).to_scipy().tolil()
+    for r in range(0, L * L, 11):
+        for q in range(1, 13):
+            c = (r + 37 * q) % (L * L)
+            A[r, c] = A[c, r] = -0.01 * q
+    A = A.tocsr()
+    A.sort_indices()
+    if cplx:
+        U = sp.triu(A, 1) * np.exp(0.3j)
+        A = (U + U.conj().T + sp.diags(A.diagonal())).tocsr()
+        A.sort_indices()
+    return ops.CSR(L * L, A.indptr.astype(np.int64), A.indices.astype(np.int32), A.data)
+
+
+# Row-sorted SELL operators, which the cooperative kernel does not take, real
+# and complex.
+@pytest.mark.parametrize("n,cplx", [(30 * 30, False), (100 * 100, False), (60 * 60, True)])
+def test_operators_the_cooperative_kernel_refuses(n, cplx, monkeypatch):
+    """After a restart the first step couples to all kept vectors; no run that
+    knows only the last two is started with it, to be thrown away."""
+    A = _uneven(n, cplx)
+    kw = dict(ned=4, maxlan=30, tol=1e-10, restart=1, maxmv=400, start=_start(A), device=True)
+    with DeviceOperator(A, fmt="sell", sigma=64) as op:
+        monkeypatch.setenv("TRLX_SPECULATE", "0")
+        seq = solve(op, **kw)
+        monkeypatch.delenv("TRLX_SPECULATE")
+        got = solve(op, **kw)
+    assert seq.info.nloop > 3
+    assert got.stats.speculative_steps > 0 and got.stats.speculative_discarded == 0
+    _same(got, seq, 4)
