@@ -22,6 +22,10 @@ REF_ROOT = os.environ.get("TRLAN_REFERENCE", "/root/reference")
 _LIB = None
 
 
+class NotBuilt(RuntimeError):
+    """The reference library is not built here (its sources are absent)."""
+
+
 def available():
     return os.path.exists(REF_SO)
 
@@ -39,7 +43,7 @@ def load():
     global _LIB
     if _LIB is None:
         if not available():
-            raise RuntimeError(f"reference oracle not built: {REF_SO}")
+            raise NotBuilt(f"reference oracle not built: {REF_SO}")
         lib = C.CDLL(REF_SO)
         declare_common(lib)
         # Internal routines used for building-block parity tests.
