@@ -856,6 +856,13 @@ def main():
                          "default for --gpus N: independent replicas")
     args = ap.parse_args()
     w = WORKLOADS[args.workload]
+    if args.impl == "reference":
+        from oracle import ref
+        if not ref.build():
+            if int(os.environ.get("RANK", "0")) == 0:
+                print(json.dumps({"impl": "reference", "unavailable": f"the reference library is not built and its "
+                                                                      f"sources are not at {ref.REF_ROOT}"}), flush=True)
+            return
     world, rank, local, pg = dist_setup(args)
     if w["kind"] == "wells":
         run_wells(args, w, world, rank, local, pg)

@@ -33,7 +33,7 @@ def available():
 def build(ref_root=None):
     """Compile the reference from its sources (only where they exist)."""
     ref_root = ref_root or REF_ROOT
-    if os.path.isdir(ref_root):
+    if os.path.isdir(os.path.join(ref_root, "SRC")):
         subprocess.run(["make", "-C", HERE, f"REF={ref_root}", "-j8"], check=True,
                        stdout=subprocess.DEVNULL)
     return available()
