@@ -35,6 +35,7 @@
 // three trips to L2 (the gather, the partial sums, the barrier, 1.2-1.5 us
 // each) and two passes over the chunk in shared memory.
 #include <algorithm>
+#include <climits>
 #include <cstdlib>
 #include <mutex>
 
@@ -105,7 +106,7 @@ __host__ __device__ constexpr size_t align16(size_t b) { return (b + 15) / 16 * 
 // Shared memory, in this order; the resident columns and entries come last.
 template <class C>
 struct Layout {
-    size_t x, y, v, z, comb, a, ad, tot, sp, ta, tb, red, col, start, count, end;
+    size_t x, y, v, z, comb, a, ad, tot, sp, ta, tb, red, col, start, count, wide, end;
     __host__ __device__ Layout(int chunk, int kmax) {
         size_t o = 0;
         auto take = [&](size_t bytes) {
@@ -128,6 +129,7 @@ struct Layout {
         col = take(sizeof(C *) * (kmax + 1));
         start = take(sizeof(int) * chunk);
         count = take(sizeof(int) * chunk);
+        wide = take(sizeof(unsigned short) * chunk);
         end = o;
     }
 };
@@ -208,10 +210,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_coop(const CoopArgs<C> A) {
     double *const red = reinterpret_cast<double *>(smem + L.red);
     C **const scol = reinterpret_cast<C **>(smem + L.col);  // the column table, columns 0 .. kmax
     int *const est = reinterpret_cast<int *>(smem + L.start), *const ecn = reinterpret_cast<int *>(smem + L.count);
+    unsigned short *const wide = reinterpret_cast<unsigned short *>(smem + L.wide);  // the block's long rows
     C *const vres = reinterpret_cast<C *>(smem + L.end);  // column c, row i at c * chunk + i
     C *const eva = vres + (size_t)A.nres * A.chunk;
     int *const eci = reinterpret_cast<int *>(eva + A.ecap);
     __shared__ int gave_up;
+    __shared__ int nwide;
     __shared__ double dd[6];    // |z|^2, Re p_k, g_k in two doubles each
     __shared__ __align__(16) double next[4];  // 1 / beta, beta^2, h_{k-1}
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -237,6 +241,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_coop(const CoopArgs<C> A) {
     const long long elast = rend > r0 ? (A.sell ? A.ptr[(rend + 31) / 32] : A.ptr[rend]) : ebase;
     const int nent = (int)(elast - ebase);
     const bool cached = nent <= A.ecap;
+    if (tid == 0) nwide = 0;
+    __syncthreads();
     for (int i = tid; i < rows; i += kThreads) {
         const long row = r0 + i;
         int st = 0, cn = 0;
@@ -252,6 +258,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_coop(const CoopArgs<C> A) {
         }
         est[i] = st;
         ecn[i] = cn;
+        if (cn > A.wide) wide[atomicAdd(&nwide, 1)] = (unsigned short)i;
         sv[i] = ldcg(A.cols[A.j0] + row);
         sx[i] = sv[i];
     }
@@ -399,36 +406,39 @@ __global__ void __launch_bounds__(kThreads, 1) k_coop(const CoopArgs<C> A) {
             const C *const gz = s > 1 ? A.z[(s - 1) & 1] : scol[A.j0];
             const C *const gv = scol[k - (s > 1 ? 1 : 0)];
             const double dl = delta;
-            const int sub = tid & (tpr - 1);
             const C *va = cached ? eva : A.va + ebase;
             const int *ci = cached ? eci : A.ci + ebase;
-            for (int i0 = 0; i0 < rows; i0 += kProductThreads / tpr) {
-                const int i = i0 + tid / tpr;
-                const bool on = i < rows && tid / tpr < kProductThreads / tpr;
-                C acc = czero(C());
-                if (on) {
+            // tpr lanes per row; then the long rows, a warp each.
+            for (int turn = 0; turn < (nwide > 0 ? 2 : 1); ++turn) {
+                const int lanes = turn ? 32 : tpr, items = turn ? nwide : rows, sub = tid & (lanes - 1);
+                for (int i0 = 0; i0 < items; i0 += kProductThreads / lanes) {
+                    const int e = i0 + tid / lanes, i = e < items ? (turn ? wide[e] : e) : 0;
                     const int st = est[i], cn = ecn[i];
-                    constexpr int U = 8 / cw;
-                    for (int t0 = sub; t0 < cn; t0 += U * tpr) {
-                        C xz[U], xv[U];
+                    const bool on = e < items && (turn || cn <= A.wide);
+                    C acc = czero(C());
+                    if (on) {
+                        constexpr int U = 8 / cw;
+                        for (int t0 = sub; t0 < cn; t0 += U * lanes) {
+                            C xz[U], xv[U];
 #pragma unroll
-                        for (int u = 0; u < U; ++u) {
-                            if (t0 + u * tpr < cn) {
-                                const int col = ci[st + (t0 + u * tpr) * estride];
-                                xz[u] = ldcg(gz + col);
-                                xv[u] = ldcg(gv + col);
+                            for (int u = 0; u < U; ++u) {
+                                if (t0 + u * lanes < cn) {
+                                    const int col = ci[st + (t0 + u * lanes) * estride];
+                                    xz[u] = ldcg(gz + col);
+                                    xv[u] = ldcg(gv + col);
+                                }
                             }
-                        }
 #pragma unroll
-                        for (int u = 0; u < U; ++u)
-                            if (t0 + u * tpr < cn)
-                                acc = acc + mulx(va[st + (t0 + u * tpr) * estride], xz[u] - dl * xv[u]);
+                            for (int u = 0; u < U; ++u)
+                                if (t0 + u * lanes < cn)
+                                    acc = acc + mulx(va[st + (t0 + u * lanes) * estride], xz[u] - dl * xv[u]);
+                        }
                     }
-                }
-                for (int o = tpr / 2; o > 0; o >>= 1) acc = acc + shfl_x(acc, o);
-                if (sub == 0 && on) {
-                    sy[i] = acc;
-                    if (s > 1) sx[i] = sz[i] - dl * sv[i];
+                    for (int o = lanes / 2; o > 0; o >>= 1) acc = acc + shfl_x(acc, o);
+                    if (sub == 0 && on) {
+                        sy[i] = acc;
+                        if (s > 1) sx[i] = sz[i] - dl * sv[i];
+                    }
                 }
             }
         } else if (s == 1) {
@@ -763,6 +773,11 @@ int launch_coop(const trlx_operator *A, C *const *cols, C *z0, C *z1, long n_pad
     a.tpr = 1;
     while (a.tpr < 32 && A->nnz > 8ll * a.tpr * A->nrow) a.tpr *= 2;
     a.sell = op_sell(A) ? 1 : 0;
+    // A row of more than four such loads gets a warp: the other rows, and with
+    // them the grid, would wait for it (lattice with one row of 3000 entries,
+    // 30000 rows, a call: 49.5 -> 4.8 ms; of 300, 7.6 -> 3.0; discrete kernels
+    // 14.3 and 7.3).  Not in SELL form, where 32 neighbouring rows are as long.
+    a.wide = a.sell || a.tpr == 32 ? INT_MAX : 32 * a.tpr;
     a.ptr = a.sell ? A->slice_ptr : A->row_ptr;
     a.ci = A->col;
     a.va = static_cast<const C *>(A->val);

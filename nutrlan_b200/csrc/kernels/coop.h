@@ -20,6 +20,7 @@ struct CoopArgs {
     const long long *ptr;  // CSR row pointers, or SELL-C-32 slice pointers
     int sell;
     int tpr;         // lanes per row of the product (a power of two)
+    int wide;        // rows of more entries get a warp
     const int *ci;
     const C *va;
     C *const *cols;  // basis column table

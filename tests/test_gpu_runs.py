@@ -79,3 +79,60 @@ def test_operators_the_cooperative_kernel_refuses(n, cplx, monkeypatch):
     assert seq.info.nloop > 3
     assert got.stats.speculative_steps > 0 and got.stats.speculative_discarded == 0
     _same(got, seq, 4)
+
+
+def _hubs(n, width, hubs, cplx=False):
+    """A band matrix of `width` entries per inner row; row r has about `deg`
+    entries more for each (r, deg) of `hubs`."""
+    import scipy.sparse as sp
+    k = width // 2
+    U = sp.diags([np.full(n - j, -1.0 / j) for j in range(1, k + 1)], list(range(1, k + 1)), shape=(n, n)).tocoo()
+    at, to = [U.row], [U.col]
+    v = [U.data]
+    for r, deg in hubs:
+        c = np.setdiff1d(np.linspace(0, n - 1, deg).astype(np.int64), [r])
+        at.append(np.minimum(r, c)), to.append(np.maximum(r, c)), v.append(np.full(c.size, -0.01))
+    U = sp.coo_matrix((np.concatenate(v), (np.concatenate(at), np.concatenate(to))), shape=(n, n)).tocsr()
+    if cplx:
+        U = U * np.exp(0.3j)
+    A = (U + U.conj().T + sp.diags(4.0 * ops.uniform01(3, np.arange(n, dtype=np.uint64)))).tocsr()
+    A.sort_indices()
+    return ops.CSR(n, A.indptr.astype(np.int64), A.indices.astype(np.int32), A.data)
+
+
+# Rows on both sides of 32 entries (one lane a row, a warp above), the first
+# and the last of all, many of them in one block; two and sixteen lanes a row;
+# entries kept in shared memory and not.
+@pytest.mark.parametrize("fmt", ["csr", "sell"])
+@pytest.mark.parametrize("n,width,hubs,cplx", [
+    (3001, 5, [(0, 27), (100, 28), (101, 29), (3000, 300)], False), (5000, 5, [(r, 40) for r in range(64, 200)], False),
+    (40000, 5, [(39999, 9000), (7, 20000)], False), (5000, 13, [(9, 59), (10, 61), (4999, 2500)], False),
+    (3000, 91, [(0, 2900), (1, 500)], False), (5000, 5, [(0, 31), (2500, 2000), (2501, 5000)], True)])
+def test_cooperative_runs_on_long_rows(n, width, hubs, cplx, fmt, monkeypatch):
+    A = _hubs(n, width, hubs, cplx)
+    kw = dict(ned=4, maxlan=24, tol=1e-13, restart=1, maxmv=60, start=_start(A), device=True)
+    with DeviceOperator(A, fmt=fmt) as op:
+        monkeypatch.setenv("TRLX_SPECULATE", "0")
+        seq = solve(op, **kw)
+        monkeypatch.delenv("TRLX_SPECULATE")
+        coop = solve(op, **kw)
+        again = solve(op, **kw)
+    assert coop.stats.speculative_steps > 0 and coop.stats.kernel_launches < seq.stats.kernel_launches / 4
+    _same(coop, seq, 4)
+    np.testing.assert_array_equal(again.eval, coop.eval)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_long_row_is_not_left_to_a_few_lanes(cplx, monkeypatch):
+    """One row of 3000 entries: a cooperative run takes no longer than the
+    discrete kernels, which give every row eight lanes."""
+    A = _hubs(30000, 5, [(15000, 3000)], cplx)
+    kw = dict(ned=4, maxlan=40, tol=1e-13, restart=1, maxmv=80, start=_start(A), device=True)
+
+    def best(op):
+        return min(solve(op, **kw).stats.seconds_total for _ in range(5))
+    with DeviceOperator(A, fmt="csr") as op:
+        coop = best(op)
+        monkeypatch.setenv("TRLX_COOP", "0")
+        discrete = best(op)
+    assert coop < discrete
