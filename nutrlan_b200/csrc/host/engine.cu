@@ -19,6 +19,7 @@
 //   * the small projected problem stays on the host in FP64.
 #include <algorithm>
 #include <cfloat>
+#include <climits>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -288,6 +289,11 @@ class Engine {
     bool sweep_off_ = false;  // a sweep's launch or memory was refused: the solve goes on without
     bool coop_off_ = false;   // the same of a cooperative run's launch
     static bool in_range(double beta) { return beta > 1e-90 && beta < 1e90; }
+    // Steps since the last one that was not taken as runs assume (INT_MAX:
+    // there was none).  A run is at most half as long, so that operators whose
+    // steps often need a second pass do not have run after run thrown away.
+    int streak_ = INT_MAX;
+    void took_steps(int n, bool as_assumed) { streak_ = !as_assumed ? 0 : streak_ > INT_MAX - n ? INT_MAX : streak_ + n; }
     bool sweeps(int jnd) const;
     bool coop_steps(int jnd, int S) const;
     size_t partial_doubles() const { return (size_t)scratch_.max_blocks * (P_ + 2) * 2; }
@@ -1401,6 +1407,7 @@ int Engine<T>::spec_segment(int *jnd_io, int S, int kept) {
     if (!(coop && h_log_[-4] != 0.0))
         while (acc < S && accept_step(j0 + acc + 1, kept, h_log_ + 4 * (acc + 1), sweep || coop)) ++acc;
     const int dropped = S - acc;
+    took_steps(acc, dropped == 0);
     spec_accepted_ += acc;
     info_->matvec -= dropped;
     discarded_ += dropped;
@@ -1682,6 +1689,7 @@ void Engine<T>::run() {
             run = std::min<long>((long)info->klan - jnd, std::max<long>(2, (long)next_test - info->matvec));
             const bool sweep = sweeps(jnd);
             if (sweep) run = std::min<long>(run, kSweepCols + 1 - jnd);
+            run = std::min<long>(run, streak_ / 2);
             if (run >= 2 && (sweep || coop_steps(jnd, (int)run))) acc = spec_segment(&jnd, (int)run, kept);
             if (acc < 0) {
                 stat = acc;
@@ -1733,7 +1741,9 @@ void Engine<T>::run() {
         }
         fl_ += 2 * jnd * nrow_ + nrow_ + nrow_;
         double f0 = fl_;
+        const int passes = info->north;
         stat = orth(jnd, false, 0.0, kept);
+        took_steps(1, info->north == passes + 1);
         fl_h_ += fl_ - f0;
         tm_end();
         if (stat) break;
@@ -1776,9 +1786,11 @@ void Engine<T>::run() {
                 if (sweep) S = std::min<long>(S, kSweepCols + 1 - jnd);
                 if (next_test > info->matvec) S = std::min<long>(S, (long)next_test - info->matvec);
                 else S = 1;
+                S = std::min<long>(S, streak_ / 2);
                 // A single step pays as a cooperative run only, the discrete
                 // kernels need a column before the last.
-                if (S >= 2 ? sweep || (kWide && jnd >= 2) || coop_steps(jnd, (int)S) : coop_steps(jnd, (int)S)) {
+                if (S >= 2 ? sweep || (kWide && jnd >= 2) || coop_steps(jnd, (int)S)
+                           : S == 1 && coop_steps(jnd, (int)S)) {
                     const int acc = spec_segment(&jnd, (int)S, kept);
                     if (acc < 0) {
                         stat = acc;
@@ -1806,7 +1818,9 @@ void Engine<T>::run() {
             tm_mid();
             fl_ += 6 * nrow_;
             double f1 = fl_;
+            const int passes = info->north;
             stat = orth(jnd, true, beta_[jnd - 2], kept);
+            took_steps(1, info->north == passes + 1);
             fl_h_ += fl_ - f1;
             tm_end();
             alfrot_[jnd - 1] = alpha_[jnd - 1];

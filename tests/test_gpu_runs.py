@@ -136,3 +136,19 @@ def test_long_row_is_not_left_to_a_few_lanes(cplx, monkeypatch):
         monkeypatch.setenv("TRLX_COOP", "0")
         discrete = best(op)
     assert coop < discrete
+
+
+# A 32-bit basis of few rows: the rounding of the stored vectors makes a second
+# pass necessary every few steps.
+@pytest.mark.parametrize("L", [6, 8, 10])
+def test_runs_shorten_where_steps_are_rejected(L, monkeypatch):
+    A = ops.anderson_3d(L, seed=5)
+    kw = dict(ned=6, maxlan=48, tol=1e-13, restart=1, maxmv=150, start=_start(A), basis_bits=32, device=True)
+    with DeviceOperator(A, fmt="csr") as op:
+        monkeypatch.setenv("TRLX_SPECULATE", "0")
+        seq = solve(op, **kw)
+        monkeypatch.delenv("TRLX_SPECULATE")
+        got = solve(op, **kw)
+    assert seq.info.north > 0 and got.stat == seq.stat == 0
+    assert got.stats.speculative_discarded <= 150 // 2      # no more than half the solve's steps
+    np.testing.assert_allclose(got.eval[:6], seq.eval[:6], rtol=1e-10)
