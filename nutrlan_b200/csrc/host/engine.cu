@@ -185,10 +185,6 @@ Options options_from(const trlx_options *o) {
 
 namespace {
 
-// FP64 and complex128 vectors shorter than this take their steps in the
-// cooperative kernel instead of sweeps.
-constexpr long kSweepMinRows = 1L << 17;
-
 enum Scal { kAlpha = 0, kR2Pre = 1, kH2 = 2, kR2Post = 3, kNorm = 4, kNumScal = 8 };
 
 double now_s() {
@@ -1107,25 +1103,26 @@ int Engine<T>::final_vectors(int jnd, int kept) {
 // For short vectors the host round trip of every Lanczos step (read alpha
 // and the norms, take trl_orth's decisions, launch the next step) costs more
 // than the step's kernels, and for long ones it is still 1-2% of a step.
-// With a built-in operator
-// the engine issues a run of steps without waiting, each assuming the
-// outcome trl_orth takes in almost every step: the full classical
-// Gram-Schmidt path with one pass (its stop test passes) and a beta that is
-// neither negligible nor a random restart.  Each step logs alpha, |r|^2
-// before and after the pass and |h|^2; the recurrence of the next step takes
-// beta = sqrt(|r|^2 after) from that log on the device, and the normalisation
-// uses the same value, so an accepted step is bitwise identical to the
-// sequential one.  The host then replays trl_orth's decisions on the logged
-// values in order; the first step whose decisions differ and everything after
-// it are discarded (their operator applications are subtracted from matvec)
-// and rerun by the sequential path.  TRLX_SPECULATE=0 disables it.
+// With a built-in operator the engine issues a run of steps without waiting,
+// each assuming the outcome trl_orth takes in almost every step: the full
+// classical Gram-Schmidt path with one pass (its stop test passes) and a beta
+// that is neither negligible nor a random restart.  Each step logs alpha,
+// |r|^2 before and after the pass and |h|^2; the recurrence of the next step
+// takes beta = sqrt(|r|^2 after) from that log on the device, and the
+// normalisation uses the same value.  The host then replays trl_orth's
+// decisions on the logged values in order; the first step whose decisions
+// differ and everything after it are discarded (their operator applications
+// are subtracted from matvec) and rerun by the sequential path.
+// TRLX_SPECULATE=0 disables it.
 //
-// A run's steps are single sweeps (sweep.h) for vectors of kSweepMinRows rows
-// or more, one cooperative kernel for shorter CSR problems, else the discrete
-// kernels (FP64/c128 basis; a shorter 32-bit basis takes its steps one by
-// one).  Sweeps and the cooperative kernel differ from the sequential path in
-// rounding only.  Measured at 2^18 rows, 128 columns: 25.1 ms a solve with
-// the discrete kernels, 11.7 with sweeps.
+// A run's steps are one cooperative kernel where that is the better one
+// (coop_pays) and applies, else single sweeps (sweep.h), else the discrete
+// kernels: FP64/c128 bases beyond the columns a sweep takes, and short
+// operators that the cooperative kernel does not take.  An accepted step of
+// the discrete kernels is bitwise the sequential one; sweeps and the
+// cooperative kernel differ from it in rounding only.
+// Measured at 2^18 rows, 128 columns: 25.1 ms a solve with the discrete
+// kernels, 11.7 with sweeps.
 template <class T>
 bool Engine<T>::spec_enabled() const {
     if (!builtin_ || uo_ || comm_ || builtin_->halo) return false;
@@ -1137,8 +1134,8 @@ bool Engine<T>::spec_enabled() const {
 // (sweep.h).
 template <class T>
 bool Engine<T>::sweeps(int jnd) const {
-    // A 32-bit basis has no other speculative steps, so any length counts.
-    if ((kWide && n_pad_ < kSweepMinRows) || jnd < 1 || jnd + 1 > kSweepCols || scale_off_ || sweep_off_)
+    // A 32-bit basis has no other speculative steps.
+    if ((kWide && coop_pays<C>(builtin_, n_pad_)) || jnd < 1 || jnd + 1 > kSweepCols || scale_off_ || sweep_off_)
         return false;
     if ((size_t)P_ * n_pad_ * sizeof(T) > (1ull << 36)) return false;  // 32-bit column offsets, 16-byte units
     const char *e = std::getenv("TRLX_SWEEP");
@@ -1149,7 +1146,7 @@ bool Engine<T>::sweeps(int jnd) const {
 template <class T>
 bool Engine<T>::coop_steps(int jnd, int S) const {
     if constexpr (kWide) {
-        if (jnd < 1 || n_pad_ >= kSweepMinRows || scale_off_ || coop_off_) return false;
+        if (jnd < 1 || !coop_pays<C>(builtin_, n_pad_) || scale_off_ || coop_off_) return false;
         const char *e = std::getenv("TRLX_COOP");
         return !(e && e[0] == '0') && coop_applies<C>(builtin_, n_pad_, jnd + S, partial_doubles());
     }

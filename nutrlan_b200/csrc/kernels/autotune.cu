@@ -90,6 +90,7 @@ void move_storage(trlx_operator *dst, trlx_operator *src) {
     std::swap(dst->sigma, src->sigma);
     std::swap(dst->slice_ptr, src->slice_ptr);
     std::swap(dst->perm, src->perm);
+    std::swap(dst->longest, src->longest);
 }
 
 // Refills the first mp columns of the basis buffer as storage type V

@@ -750,6 +750,12 @@ bool make_plan(const trlx_operator *A, long n_pad, int kmax, size_t part_doubles
 }  // namespace
 
 template <class C>
+bool coop_pays(const trlx_operator *A, long n_pad) {
+    const long long words = cwidth<C>() * A->nnz;
+    return n_pad < kCoopRows && (words <= kCoopWords || words < (op_sell(A) ? 16384ll : 512ll) * A->longest);
+}
+
+template <class C>
 bool coop_applies(const trlx_operator *A, long n_pad, int kmax, size_t part_doubles) {
     Plan p;
     return make_plan<C>(A, n_pad, kmax, part_doubles, &p);
@@ -808,6 +814,8 @@ int launch_coop(const trlx_operator *A, C *const *cols, C *z0, C *z1, long n_pad
     return -1;
 }
 
+template bool coop_pays<double>(const trlx_operator *, long);
+template bool coop_pays<zd>(const trlx_operator *, long);
 template bool coop_applies<double>(const trlx_operator *, long, int, size_t);
 template bool coop_applies<zd>(const trlx_operator *, long, int, size_t);
 template int launch_coop<double>(const trlx_operator *, double *const *, double *, double *, long, int, int, int,

@@ -35,6 +35,29 @@ struct CoopArgs {
     long polls;      // of the grid barrier before it gives up
 };
 
+// Operators of at least so many rows take their steps as sweeps (sweep.h):
+// the basis leaves L2, and the cooperative kernel reads it twice a step.
+// Lattice, 5 entries a row, cooperative / sweeps, a call: 123904 rows, 48
+// columns 3.3 / 3.7 ms, 96 columns 5.4 / 6.0; 186624 rows 4.3 / 4.2, 9.2 / 7.0.
+// (Complex: 65536 rows 3.4 / 4.5 and 6.3 / 7.2, 92416 rows 4.8 / 4.5 and 11.7 / 7.6;
+// four launches a step 7.6 and 13.1.)
+constexpr long kCoopRows = 1L << 17;
+// So do operators of more doubles than this to gather in a product: the
+// cooperative kernel gathers from two vectors.  Random columns, 48 columns,
+// cooperative / sweeps / four launches a step, a call: 98304 rows of 17
+// entries 6.3 / 4.9 / 6.8 ms, of 33 9.4 / 6.0 / 8.5, of 65 20.1 / 11.3 / 13.7;
+// 32768 rows of 33 3.3 / 3.7 / 5.5, of 129 7.1 / 5.0 / 6.8.  (Band matrices
+// lose some there: 98304 rows of 33, 64 columns, 5.4 / 6.5 / 9.0.)
+constexpr long long kCoopWords = 1500000;
+
+// Whether a run of this operator is better off in the cooperative kernel than
+// in sweeps, by rows and entries.  The product kernels that sweeps alternate
+// with leave a row to one lane (SELL) or eight (CSR), so that a long row
+// outweighs the second gather: 98304 rows of 33 entries, one of 3000 12.5 /
+// 10.2 ms, of 10000 15.6 / 18.2; SELL, 17 entries, longest 300 8.5 / 16.3.
+template <class C>
+bool coop_pays(const trlx_operator *A, long n_pad);
+
 constexpr long kCoopPolls = 1L << 22;  // some seconds
 
 // Whether the kernel takes runs of this operator, up to `kmax` columns, on the

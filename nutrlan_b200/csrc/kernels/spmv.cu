@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../../include/trlx.h"
+#include "coop.h"
 #include "spmv.h"
 #include "../host/comm.h"
 #include "../host/hostcopy.h"
@@ -553,6 +554,27 @@ std::vector<X> to_host(const X *src, size_t count, int where) {
     return h;
 }
 
+// Entries of the longest row, for the operators whose steps it decides the
+// form of (coop_pays); 0 for the others and where it cannot be had.
+int longest_row(int nrow, const long long *rp, long long nnz, int cw, int where) {
+    if (nrow >= trlb::kCoopRows || cw * nnz <= trlb::kCoopWords) return 0;
+    const int nslice = (nrow + 31) / 32;
+    std::vector<int> w(nslice, 0);
+    if (where == TRLX_DEVICE_ARRAYS) {
+        int *d_w = nullptr;
+        if (op_alloc(reinterpret_cast<void **>(&d_w), sizeof(int) * nslice) == cudaSuccess) {
+            trlb::launch_slice_width(nrow, nslice, rp, nullptr, d_w, trlb::sell_build_grid(nslice));
+            if (cudaMemcpy(w.data(), d_w, sizeof(int) * nslice, cudaMemcpyDeviceToHost) != cudaSuccess)
+                std::fill(w.begin(), w.end(), 0);
+            op_free(d_w);
+        }
+        cudaGetLastError();
+    } else {
+        for (int i = 0; i < nrow; ++i) w[i / 32] = std::max(w[i / 32], (int)(rp[i + 1] - rp[i]));
+    }
+    return *std::max_element(w.begin(), w.end());
+}
+
 int check_csr(int nrow, const long long *rp, const int *ci, const void *val) {
     if (nrow <= 0 || !rp || !ci || !val) return -1;
     return 0;
@@ -577,6 +599,7 @@ extern "C" int trlx_csr_create(int nrow, const long long *row_ptr, const int *co
     if (!rc) rc = to_device(col_idx, (size_t)nnz, where, &A->col);
     double *dv = nullptr;
     if (!rc) rc = to_device(val, (size_t)nnz, where, &dv);
+    if (!rc) A->longest = longest_row(nrow, row_ptr, nnz, 1, where);
     A->val = dv;
     if (rc) {
         trlx_operator_destroy(A);
@@ -603,6 +626,7 @@ extern "C" int trlx_zcsr_create(int nrow, const long long *row_ptr, const int *c
     if (!rc) rc = to_device(col_idx, (size_t)nnz, where, &A->col);
     trlb::zd *dv = nullptr;
     if (!rc) rc = to_device(reinterpret_cast<const trlb::zd *>(val), (size_t)nnz, where, &dv);
+    if (!rc) A->longest = longest_row(nrow, row_ptr, nnz, 2, where);
     A->val = dv;
     if (rc) {
         trlx_operator_destroy(A);
@@ -670,7 +694,10 @@ int sell_create(int nrow, const long long *row_ptr, const int *col_idx, const V 
         trlb::launch_slice_width(nrow, nslice, d_rp, A->perm, d_w, grid);
         std::vector<int> w(nslice);
         if (cudaMemcpy(w.data(), d_w, sizeof(int) * nslice, cudaMemcpyDeviceToHost) != cudaSuccess) rc = -3;
-        for (int s = 0; s < nslice && !rc; ++s) sp[s + 1] = sp[s] + 32LL * w[s];
+        for (int s = 0; s < nslice && !rc; ++s) {
+            sp[s + 1] = sp[s] + 32LL * w[s];
+            A->longest = std::max(A->longest, w[s]);
+        }
     }
     if (!rc) rc = to_device(sp.data(), sp.size(), TRLX_HOST_ARRAYS, &A->slice_ptr);
     const long long total = sp[nslice];

@@ -26,6 +26,7 @@ struct trlx_operator {
     int sigma = 1;
     long long *slice_ptr = nullptr;  // offset of slice s (entries), nslice+1
     int *perm = nullptr;             // stored row -> original row (nullptr = identity)
+    int longest = 0;  // entries of the longest row (CSR: 0 where coop_pays needs none)
     int device = -1;
     // Block-row distribution (trlx_dist_*_create): columns [0, nrow) are
     // this rank's rows, [nrow, nrow + halo entries) values received from

@@ -1,6 +1,8 @@
 """Runs of Lanczos steps that are issued ahead of the host's decisions, where
 they go wrong or do not apply: the solve goes on with the sequential steps
 (trl_orth's decisions, SRC/trlcore.c:2913-3117) and gives what those give."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -152,3 +154,65 @@ def test_runs_shorten_where_steps_are_rejected(L, monkeypatch):
     assert seq.info.north > 0 and got.stat == seq.stat == 0
     assert got.stats.speculative_discarded <= 150 // 2      # no more than half the solve's steps
     np.testing.assert_allclose(got.eval[:6], seq.eval[:6], rtol=1e-10)
+
+
+def _random(n, per, cplx=False, longest=0):
+    """About `per` entries a row in random columns; row 0 with `longest`."""
+    import scipy.sparse as sp
+    rng = np.random.default_rng(1)
+    m = n * (per - 1) // 2
+    i, j, v = rng.integers(0, n, m), rng.integers(0, n, m), rng.standard_normal(m)
+    if longest:
+        c = rng.choice(np.arange(1, n), longest, replace=False)
+        i, j, v = np.concatenate([i, np.zeros_like(c)]), np.concatenate([j, c]), np.concatenate([v, np.full(longest, -0.01)])
+    U = sp.triu(sp.coo_matrix((np.concatenate([v, v]), (np.concatenate([i, j]), np.concatenate([j, i]))), shape=(n, n)).tocsr(), 1)
+    if cplx:
+        U = U * np.exp(0.3j)
+    A = (U + U.conj().T + sp.diags(rng.standard_normal(n))).tocsr()
+    A.sort_indices()
+    return ops.CSR(n, A.indptr.astype(np.int64), A.indices.astype(np.int32), A.data)
+
+
+# Operators on both sides of the lines between cooperative runs (one launch for
+# many steps) and sweeps (two a step): doubles to gather in a product, and the
+# longest row against them.
+@pytest.mark.parametrize("device", [False, True])
+@pytest.mark.parametrize("n,per,cplx,longest,fmt,one", [
+    (30000, 49, False, 0, "csr", True), (30000, 53, False, 0, "csr", False), (15000, 49, True, 0, "csr", True),
+    (15000, 53, True, 0, "csr", False), (30000, 65, False, 6000, "csr", True), (30000, 65, False, 0, "sell", False),
+    (30000, 65, False, 900, "sell", True)])
+def test_steps_of_operators_with_many_entries(n, per, cplx, longest, fmt, one, device, monkeypatch):
+    A = _random(n, per, cplx, longest)
+    kw = dict(ned=4, maxlan=24, tol=1e-13, restart=1, maxmv=60, start=_start(A), device=True)
+    with DeviceOperator(A, fmt=fmt) as op:
+        if device:      # the same operator from arrays on the device
+            import torch
+            arrays = [torch.as_tensor(a).cuda() for a in (A.row_ptr, A.col, A.val)]
+            op.close()
+            create = getattr(op.lib, f"trlx_{op.fmt}_create")
+            args = [n, *(a.data_ptr() for a in arrays)] + ([1] if fmt == "sell" else [])
+            assert create(*args, 1, C.byref(op.handle)) == 0
+        monkeypatch.setenv("TRLX_SPECULATE", "0")
+        seq = solve(op, **kw)
+        monkeypatch.delenv("TRLX_SPECULATE")
+        got = solve(op, **kw)
+    assert got.stats.speculative_steps > 0 and got.stats.speculative_discarded == 0
+    assert (got.stats.kernel_launches < 60) == one
+    _same(got, seq, 4)
+
+
+@pytest.mark.parametrize("fmt", ["csr", "sell"])
+def test_many_entries_are_not_gathered_twice(fmt, monkeypatch):
+    """65536 rows of 65 entries: steps take no longer than with the discrete
+    kernels."""
+    A = _random(65536, 65)
+    kw = dict(ned=4, maxlan=40, tol=1e-13, restart=1, maxmv=80, start=_start(A), device=True)
+
+    def best(op):
+        return min(solve(op, **kw).stats.seconds_total for _ in range(5))
+    with DeviceOperator(A, fmt=fmt) as op:
+        got = best(op)
+        monkeypatch.setenv("TRLX_COOP", "0")
+        monkeypatch.setenv("TRLX_SWEEP", "0")
+        discrete = best(op)
+    assert got < discrete
