@@ -285,11 +285,14 @@ class Engine {
     bool sweep_off_ = false;  // a sweep's launch or memory was refused: the solve goes on without
     bool coop_off_ = false;   // the same of a cooperative run's launch
     static bool in_range(double beta) { return beta > 1e-90 && beta < 1e90; }
-    // Steps since the last one that was not taken as runs assume (INT_MAX:
-    // there was none).  A run is at most half as long, so that operators whose
-    // steps often need a second pass do not have run after run thrown away.
+    // Steps since the last one that was not taken as runs assume, once a run
+    // was cut short by one (INT_MAX before).  A run is at most half as long, so
+    // that operators whose steps often need a second pass do not have run after
+    // run thrown away.
     int streak_ = INT_MAX;
-    void took_steps(int n, bool as_assumed) { streak_ = !as_assumed ? 0 : streak_ > INT_MAX - n ? INT_MAX : streak_ + n; }
+    void took_steps(int n, bool as_assumed) {
+        if (streak_ < INT_MAX) streak_ = !as_assumed ? 0 : streak_ > INT_MAX - n ? INT_MAX : streak_ + n;
+    }
     bool sweeps(int jnd) const;
     bool coop_steps(int jnd, int S) const;
     size_t partial_doubles() const { return (size_t)scratch_.max_blocks * (P_ + 2) * 2; }
@@ -1404,7 +1407,10 @@ int Engine<T>::spec_segment(int *jnd_io, int S, int kept) {
     if (!(coop && h_log_[-4] != 0.0))
         while (acc < S && accept_step(j0 + acc + 1, kept, h_log_ + 4 * (acc + 1), sweep || coop)) ++acc;
     const int dropped = S - acc;
-    took_steps(acc, dropped == 0);
+    if (dropped)
+        streak_ = 0;
+    else
+        took_steps(S, true);
     spec_accepted_ += acc;
     info_->matvec -= dropped;
     discarded_ += dropped;
