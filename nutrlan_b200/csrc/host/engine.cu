@@ -129,14 +129,22 @@ struct Workspace {
         pool_bytes = fbuf_bytes = small_bytes = partial_bytes = 0;
         device = -1;
     }
-    // Grows buf to at least `bytes`; returns false on allocation failure.
-    static bool ensure(void **buf, size_t *have, size_t bytes) {
+    // Grows buf to at least `bytes`; returns false on allocation failure.  The
+    // vectors kept for runs make way: they only save time.
+    bool ensure(void **buf, size_t *have, size_t bytes) {
         if (*have >= bytes && *buf) return true;
         cudaFree(*buf);
         *buf = nullptr;
         *have = 0;
         if (bytes == 0) return true;
-        if (cudaMalloc(buf, bytes) != cudaSuccess) {
+        cudaError_t e = cudaMalloc(buf, bytes);
+        if (e != cudaSuccess && saved) {
+            cudaFree(saved);
+            saved = nullptr;
+            saved_bytes = 0;
+            e = cudaMalloc(buf, bytes);
+        }
+        if (e != cudaSuccess) {
             cudaGetLastError();
             *buf = nullptr;
             return false;
@@ -508,7 +516,7 @@ int Engine<T>::setup() {
     const double t_alloc0 = now_s();
     Workspace &ws = workspace();
     const size_t pool_bytes = (size_t)P_ * n_pad_ * sizeof(T);
-    if (!Workspace::ensure(&ws.pool, &ws.pool_bytes, pool_bytes)) {
+    if (!ws.ensure(&ws.pool, &ws.pool_bytes, pool_bytes)) {
         ws.release();
         std::fprintf(stderr, "TRLAN-B200: cannot allocate %.2f GB basis pool.\n", pool_bytes / 1e9);
         return -5;
@@ -526,7 +534,7 @@ int Engine<T>::setup() {
     for (int i = 0; i < P_; ++i) lslot_[i] = i;
     h_cols_.resize(P_);
     if (!kWide) {
-        if (!Workspace::ensure(&ws.fbuf, &ws.fbuf_bytes, 3 * sizeof(C) * n_pad_)) return -5;
+        if (!ws.ensure(&ws.fbuf, &ws.fbuf_bytes, 3 * sizeof(C) * n_pad_)) return -5;
         for (int k = 0; k < 3; ++k) fbuf_[k] = static_cast<C *>(ws.fbuf) + (size_t)k * n_pad_;
         CK(cudaMemsetAsync(ws.fbuf, 0, 3 * sizeof(C) * n_pad_, st_));
         qa64_ = fbuf_[0];
@@ -538,7 +546,7 @@ int Engine<T>::setup() {
     const size_t log_len = 4 * ((size_t)maxlan_ + 2), b_coef = al(sizeof(double) * (sweep_doubles() + log_len)),
                  b_scal = al(sizeof(double) * kNumScal), b_Y = al(sizeof(double) * (size_t)maxlan_ * maxlan_),
                  b_cols = al(sizeof(T *) * P_);
-    if (!Workspace::ensure(&ws.small, &ws.small_bytes, b_coef + b_scal + b_Y + b_cols)) return -5;
+    if (!ws.ensure(&ws.small, &ws.small_bytes, b_coef + b_scal + b_Y + b_cols)) return -5;
     char *sp = static_cast<char *>(ws.small);
     d_coef_ = reinterpret_cast<C *>(sp);
     d_sc_c_ = d_coef_ + P_;
@@ -565,7 +573,7 @@ int Engine<T>::setup() {
     h_scal_ = ws.h_scal;
     scratch_.max_blocks = 148 * 8;
     scratch_.max_cols = P_;
-    if (!Workspace::ensure(&ws.partials, &ws.partial_bytes,
+    if (!ws.ensure(&ws.partials, &ws.partial_bytes,
                            (size_t)scratch_.max_blocks * (P_ + 2) * sizeof(zd)))
         return -5;
     scratch_.partials = ws.partials;
@@ -1071,8 +1079,7 @@ int Engine<T>::final_vectors(int jnd, int kept) {
         out = reinterpret_cast<C *>(evec_);
     } else {
         Workspace &ws = workspace();
-        if (!Workspace::ensure(&ws.out, &ws.out_bytes, sizeof(C) * (size_t)n_pad_ * std::max(kept, 1)))
-            return -5;
+        if (!ws.ensure(&ws.out, &ws.out_bytes, sizeof(C) * (size_t)n_pad_ * std::max(kept, 1))) return -5;
         tmp = static_cast<C *>(ws.out);
         out = tmp;
         ldo = n_pad_;
@@ -1336,7 +1343,7 @@ int Engine<T>::spec_segment(int *jnd_io, int S, int kept) {
     if (!done && sweeps(j0)) {
         if constexpr (!kWide) {
             Workspace &ws = workspace();
-            if (!Workspace::ensure(&ws.saved, &ws.saved_bytes, 2 * vec)) {
+            if (!ws.ensure(&ws.saved, &ws.saved_bytes, 2 * vec)) {
                 sweep_off_ = true;  // no memory for them: steps one by one
                 return 0;
             }
@@ -1478,7 +1485,7 @@ int Engine<T>::refine_fp64(int k, double *max_res) {
     // then G, H, the combination coefficients, the residual coefficients,
     // |r|^2, a scalar pair and 3k column pointers (all in units of C).
     const size_t elems = (2 * (size_t)k + 4) * vec + 2 * kk + 2 * kk + (size_t)k + 8 + 3 * (size_t)k;
-    if (!Workspace::ensure(&ws.refine, &ws.refine_bytes, elems * sizeof(C))) return -5;
+    if (!ws.ensure(&ws.refine, &ws.refine_bytes, elems * sizeof(C))) return -5;
     C *base = static_cast<C *>(ws.refine);
     CK(cudaMemsetAsync(base, 0, elems * sizeof(C), st_));
     C *Wb = base, *AWb = Wb + k * vec, *y0 = AWb + k * vec, *y1 = y0 + vec, *ay = y1 + vec, *zero = ay + vec;

@@ -5,6 +5,7 @@
 
 #include <cstdlib>
 #include <cstring>
+#include <unordered_map>
 
 extern "C" {
 int fake_device, fake_attribute_answer;
@@ -13,6 +14,8 @@ int fake_launches;        // how many of those were asked for
 int fake_sync_failures;   // so many waits fail after the first of those launches
 void (*fake_on_occupancy)(int call);  // called by the occupancy query of clusters, with its number
 int fake_occupancy_calls;
+size_t fake_used, fake_peak;  // bytes of device memory
+size_t fake_limit;            // the most that can be had (0: any)
 
 static void *ones(size_t bytes) {
     double *p = (double *)malloc(bytes + 256);
@@ -51,17 +54,35 @@ cudaError_t cudaLaunchKernel(const void *, dim3, dim3, void **, size_t, cudaStre
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t) { return "refused by the test"; }
 
+static std::unordered_map<void *, size_t> &sizes() {
+    static auto *m = new std::unordered_map<void *, size_t>;
+    return *m;
+}
 cudaError_t cudaMalloc(void **p, size_t n) {
+    if (fake_limit && fake_used + n > fake_limit) return cudaErrorMemoryAllocation;
     *p = ones(n);
+    sizes()[*p] = n;
+    fake_used += n;
+    if (fake_used > fake_peak) fake_peak = fake_used;
     return cudaSuccess;
 }
 cudaError_t cudaFree(void *p) {
+    if (p) {
+        fake_used -= sizes()[p];
+        sizes().erase(p);
+    }
     free(p);
     return cudaSuccess;
 }
-cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { return cudaMalloc(p, n); }
-cudaError_t cudaMallocHost(void **p, size_t n) { return cudaMalloc(p, n); }
-cudaError_t cudaFreeHost(void *p) { return cudaFree(p); }
+cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) {
+    *p = ones(n);
+    return cudaSuccess;
+}
+cudaError_t cudaMallocHost(void **p, size_t n) { return cudaHostAlloc(p, n, 0); }
+cudaError_t cudaFreeHost(void *p) {
+    free(p);
+    return cudaSuccess;
+}
 cudaError_t cudaMallocFromPoolAsync(void **p, size_t n, cudaMemPool_t, cudaStream_t) { return cudaMalloc(p, n); }
 cudaError_t cudaFreeAsync(void *p, cudaStream_t) { return cudaFree(p); }
 cudaError_t cudaMemPoolCreate(cudaMemPool_t *, const cudaMemPoolProps *) { return cudaSuccess; }

@@ -37,7 +37,7 @@ def fake(tmp_path_factory):
     return lib
 
 
-def _solve(fake, n, bits, launch_answer=0, sync_failures=0):
+def _solve(fake, n, bits, launch_answer=0, sync_failures=0, maxlan=24):
     """info.stat of a solve on a diagonal operator; the number of runs asked for."""
     def var(name):
         return C.c_int.in_dll(fake, "fake_" + name)
@@ -47,7 +47,7 @@ def _solve(fake, n, bits, launch_answer=0, sync_failures=0):
     P = lambda a: C.c_void_p(a.ctypes.data)
     assert fake.trlx_csr_create(n, P(rp), P(ci), P(va), 0, C.byref(op)) == 0
     info = TrlInfo()
-    fake.trl_init_info(C.byref(info), n, 24, -1, 3, C.c_double(1e-9), 1, 40, None)
+    fake.trl_init_info(C.byref(info), n, maxlan, -1, 3, C.c_double(1e-9), 1, 40, None)
     info.verbose, info.mvparam = -1, op.value
     fake.trl_set_iguess(C.byref(info), 0, 1, 0, None)
     ev, vec, o = np.zeros(4), np.ones((4, n)), TrlxOptions(basis_bits=bits, refine=0)
@@ -68,3 +68,23 @@ def test_error_in_a_run_is_the_solves_status(fake, n, bits):
 def test_refused_launch_leaves_the_sequential_steps(fake, n, bits):
     stat, runs = _solve(fake, n, bits, launch_answer=701)
     assert runs > 0 and stat != -1001
+
+
+def test_memory_for_runs_is_given_back_to_a_larger_solve(fake, monkeypatch):
+    """The two vectors that a run of sweeps over a 32-bit basis goes back to are
+    kept for the next solve, but not against its basis."""
+    def size(name):
+        return C.c_size_t.in_dll(fake, "fake_" + name)
+    fake.trlx_release_workspace()
+    size("peak").value = size("used").value
+    monkeypatch.setenv("TRLX_SWEEP", "0")
+    assert _solve(fake, 3000, 32, maxlan=60)[0] != -5
+    need = size("peak").value               # without those vectors
+    monkeypatch.delenv("TRLX_SWEEP")
+    fake.trlx_release_workspace()
+    assert _solve(fake, 3000, 32)[1] > 0    # the smaller solve takes sweeps
+    size("limit").value = need
+    try:
+        assert _solve(fake, 3000, 32, maxlan=60)[0] != -5
+    finally:
+        size("limit").value = 0
