@@ -11,6 +11,14 @@
 #include <vector>
 
 #include "dense_core.h"
+
+// On x86 the wide form of a vector loop is chosen when the library is loaded;
+// elsewhere the compiler's target has its vectors anyway.
+#if defined(__x86_64__) || defined(__i386__)
+#define TRLB_WIDE __attribute__((target_clones("avx512f", "avx2", "default")))
+#else
+#define TRLB_WIDE
+#endif
 #include "restart_core.h"
 
 namespace trlb {
@@ -130,8 +138,7 @@ typedef double Rows8 __attribute__((vector_size(64), aligned(8)));
 // eight rows cover the latency of a rotation's dependent multiply and add
 // (two took 2.0 ms where four take 1.1, at 128 columns).  ld is a multiple of
 // the block.
-__attribute__((target_clones("avx512f", "avx2", "default"))) void apply_sweep(int l, int m, const double *cs,
-                                                                              const double *sn, double *Z, int ld) {
+TRLB_WIDE void apply_sweep(int l, int m, const double *cs, const double *sn, double *Z, int ld) {
     constexpr int V = kRowBlock / 8;
     for (int r0 = 0; r0 < ld; r0 += kRowBlock) {
         Rows8 t[V];
