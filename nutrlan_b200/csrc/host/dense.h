@@ -74,7 +74,6 @@ class TridiagVectors {
     // For the wanted values lambda[0..nlam): yy (nd x nlam, nd = size of the
     // solved problem), with rot (nrot x nrot) applied to the first nrot rows.
     void vectors(int nrot, const double *rot, int nlam, const double *lambda, double *yy) const;
-    int size() const { return n_; }
 
    private:
     int n_ = 0, ld_ = 0;

@@ -216,3 +216,42 @@ def test_many_entries_are_not_gathered_twice(fmt, monkeypatch):
         monkeypatch.setenv("TRLX_SWEEP", "0")
         discrete = best(op)
     assert got < discrete
+
+
+# Rows that are no multiple of 256: what a rejected run leaves in the padding
+# rows of the columns (its scale is no number) does not reach a result.
+@pytest.mark.parametrize("n,bits", [((1 << 17) + 77, 64), (3001, 64), (5003, 32)])
+@pytest.mark.parametrize("fmt", ["csr", "sell"])
+def test_exhausted_basis_with_padding_rows(n, bits, fmt, monkeypatch):
+    A = ops.CSR(n, np.arange(n + 1, dtype=np.int64), np.arange(n, dtype=np.int32), 1.0 + (np.arange(n) % 6))
+    kw = dict(ned=3, maxlan=24, tol=1e-9, restart=1, maxmv=400, start=ops.start_vector(n), basis_bits=bits, device=True)
+    with DeviceOperator(A, fmt=fmt) as op:
+        r = solve(op, **kw)
+        B = ops.anderson_3d(17, seed=5)             # the same workspace after it
+        kw.update(start=_start(B), maxmv=60, maxlan=24, tol=1e-13)
+        with DeviceOperator(B, fmt=fmt) as op2:
+            after = solve(op2, **kw)
+            monkeypatch.setenv("TRLX_SPECULATE", "0")
+            seq = solve(op2, **kw)
+    assert r.stat == 0 and r.nec >= 3 and r.stats.speculative_discarded > 0
+    np.testing.assert_allclose(r.eval[:3], 1.0, rtol=1e-9)
+    np.testing.assert_allclose(after.eval[:3], seq.eval[:3], rtol=1e-12 if bits == 64 else 1e-10)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 5, 8, 12])
+@pytest.mark.parametrize("bits", [64, 32])
+def test_runs_on_the_smallest_problems(n, bits, monkeypatch):
+    """The basis spans the whole space before a run ends."""
+    import scipy.sparse as sp
+    M = sp.diags([np.arange(1.0, n + 1), np.full(n - 1, -0.5), np.full(n - 1, -0.5)], [0, 1, -1], format="csr")
+    M.sort_indices()
+    A = ops.CSR(n, M.indptr.astype(np.int64), M.indices.astype(np.int32), M.data)
+    kw = dict(ned=1, maxlan=max(n, 3), tol=1e-10, restart=1, maxmv=60, start=np.ones(n), basis_bits=bits, device=True)
+    with DeviceOperator(A) as op:
+        monkeypatch.setenv("TRLX_SPECULATE", "0")
+        seq = solve(op, **kw)
+        monkeypatch.delenv("TRLX_SPECULATE")
+        got = solve(op, **kw)
+    assert got.stat == seq.stat and got.nec == seq.nec
+    if seq.nec:
+        np.testing.assert_allclose(got.eval[:1], seq.eval[:1], rtol=1e-9)
