@@ -283,12 +283,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_coop(const CoopArgs<C> A) {
                 if (u < cn) vres[(size_t)(c + u) * chunk + i] = t[u];
         }
     }
-    // In the product A.tpr lanes per row, in the pass column slices.
-    const int tpr = A.tpr;
+    // In the pass column slices.
     const int slices = max(1, kThreads / chunk);
     const int sl = slices > 1 ? tid / chunk : 0;
     __syncthreads();
 
+    const int nw = nwide;
     double sigma = ta[A.j0 - 1], delta = 0.0;
     unsigned meets = 0;
     // Adds the clusters' partial sums of the step that made column k (into
@@ -408,11 +408,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_coop(const CoopArgs<C> A) {
             const double dl = delta;
             const C *va = cached ? eva : A.va + ebase;
             const int *ci = cached ? eci : A.ci + ebase;
-            // tpr lanes per row; then the long rows, a warp each.
-            for (int turn = 0; turn < (nwide > 0 ? 2 : 1); ++turn) {
-                const int lanes = turn ? 32 : tpr, items = turn ? nwide : rows, sub = tid & (lanes - 1);
-                for (int i0 = 0; i0 < items; i0 += kProductThreads / lanes) {
-                    const int e = i0 + tid / lanes, i = e < items ? (turn ? wide[e] : e) : 0;
+            // 2^A.lanes lanes per row; then the long rows, a warp each.
+            for (int turn = 0; turn < (nw > 0 ? 2 : 1); ++turn) {
+                const int lg = turn ? 5 : A.lanes, lanes = 1 << lg, items = turn ? nw : rows, sub = tid & (lanes - 1);
+                for (int i0 = 0; i0 < items; i0 += kProductThreads >> lg) {
+                    const int e = i0 + (tid >> lg), i = e < items ? (turn ? wide[e] : e) : 0;
                     const int st = est[i], cn = ecn[i];
                     const bool on = e < items && (turn || cn <= A.wide);
                     C acc = czero(C());
@@ -776,14 +776,14 @@ int launch_coop(const trlx_operator *A, C *const *cols, C *z0, C *z1, long n_pad
     a.chunk = p.chunk;
     // Lanes per row: one while a row's entries are loaded together anyway
     // (neighbouring rows of a lattice then read neighbouring values).
-    a.tpr = 1;
-    while (a.tpr < 32 && A->nnz > 8ll * a.tpr * A->nrow) a.tpr *= 2;
+    a.lanes = 0;
+    while (a.lanes < 5 && A->nnz > (8ll << a.lanes) * A->nrow) ++a.lanes;
     a.sell = op_sell(A) ? 1 : 0;
     // A row of more than four such loads gets a warp: the other rows, and with
     // them the grid, would wait for it (lattice with one row of 3000 entries,
     // 30000 rows, a call: 49.5 -> 4.8 ms; of 300, 7.6 -> 3.0; discrete kernels
     // 14.3 and 7.3).  Not in SELL form, where 32 neighbouring rows are as long.
-    a.wide = a.sell || a.tpr == 32 ? INT_MAX : 32 * a.tpr;
+    a.wide = a.sell || a.lanes == 5 ? INT_MAX : 32 << a.lanes;
     a.ptr = a.sell ? A->slice_ptr : A->row_ptr;
     a.ci = A->col;
     a.va = static_cast<const C *>(A->val);

@@ -19,7 +19,7 @@ struct CoopArgs {
     int ecap;        // operator entries kept in shared memory per block (0: none)
     const long long *ptr;  // CSR row pointers, or SELL-C-32 slice pointers
     int sell;
-    int tpr;         // lanes per row of the product (a power of two)
+    int lanes;       // log2 of the lanes per row of the product
     int wide;        // rows of more entries get a warp
     const int *ci;
     const C *va;
