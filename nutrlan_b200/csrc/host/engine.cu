@@ -1707,57 +1707,57 @@ void Engine<T>::run() {
             }
         }
         if (acc == 0) {
-        // ---- first step after (re)start: arrowhead coupling -------------------
-        jnd++;
-        if (jnd + 1 > maxlan_ + 1 || jnd + 1 >= P_) {
-            stat = -1111;
-            break;
-        }
-        // FP64 views of the current vector and the output slot.
-        if constexpr (kWide) {
-            qa64_ = reinterpret_cast<C *>(col(jnd - 1));
-            qb64_ = jnd >= 2 ? reinterpret_cast<C *>(col(jnd - 2)) : nullptr;
-            r64_ = reinterpret_cast<C *>(col(jnd));
-        }
-        tm_begin();
-        if ((stat = apply_op(qa64_, r64_, true))) break;
-        tm_mid();
-        // Coefficients (beta_0 .. beta_{jnd-2}, alpha_{jnd-1}); the device
-        // writes alpha into the last slot before the coupling update.
-        {
-            std::vector<C> g(jnd);
-            for (int i = 0; i < jnd - 1; ++i) {
-                if constexpr (kComplex)
-                    g[i] = zd{beta_[i], 0.0};
-                else
-                    g[i] = beta_[i];
-            }
-            if constexpr (kComplex)
-                g[jnd - 1] = zd{0.0, 0.0};
-            else
-                g[jnd - 1] = 0.0;
-            if (cudaMemcpyAsync(d_coef_, g.data(), sizeof(C) * jnd, cudaMemcpyHostToDevice, st_) != cudaSuccess) {
-                stat = -1001;
+            // ---- first step after (re)start: arrowhead coupling -------------------
+            jnd++;
+            if (jnd + 1 > maxlan_ + 1 || jnd + 1 >= P_) {
+                stat = -1111;
                 break;
             }
-            cudaMemcpyAsync(reinterpret_cast<double *>(d_coef_ + (jnd - 1)), d_scal_ + kAlpha, sizeof(double),
-                            cudaMemcpyDeviceToDevice, st_);
-            Recur<C> none;
-            int pid = pbeg();
-            launch_update<T>(d_cols_, jnd, n_pad_, r64_, none, d_coef_, r64_, d_scal_ + kR2Post, scratch_, st_);
-            pend(pid, TRLX_K_UPDATE, (double)jnd * nrow_ * sv() + 2.0 * nrow_ * cs());
-            count_launch();
-            cudaStreamSynchronize(st_);  // g must outlive the copy
-        }
-        fl_ += 2 * jnd * nrow_ + nrow_ + nrow_;
-        double f0 = fl_;
-        const int passes = info->north;
-        stat = orth(jnd, false, 0.0, kept);
-        took_steps(1, info->north == passes + 1);
-        fl_h_ += fl_ - f0;
-        tm_end();
-        if (stat) break;
-        rotate_fp64();
+            // FP64 views of the current vector and the output slot.
+            if constexpr (kWide) {
+                qa64_ = reinterpret_cast<C *>(col(jnd - 1));
+                qb64_ = jnd >= 2 ? reinterpret_cast<C *>(col(jnd - 2)) : nullptr;
+                r64_ = reinterpret_cast<C *>(col(jnd));
+            }
+            tm_begin();
+            if ((stat = apply_op(qa64_, r64_, true))) break;
+            tm_mid();
+            // Coefficients (beta_0 .. beta_{jnd-2}, alpha_{jnd-1}); the device
+            // writes alpha into the last slot before the coupling update.
+            {
+                std::vector<C> g(jnd);
+                for (int i = 0; i < jnd - 1; ++i) {
+                    if constexpr (kComplex)
+                        g[i] = zd{beta_[i], 0.0};
+                    else
+                        g[i] = beta_[i];
+                }
+                if constexpr (kComplex)
+                    g[jnd - 1] = zd{0.0, 0.0};
+                else
+                    g[jnd - 1] = 0.0;
+                if (cudaMemcpyAsync(d_coef_, g.data(), sizeof(C) * jnd, cudaMemcpyHostToDevice, st_) != cudaSuccess) {
+                    stat = -1001;
+                    break;
+                }
+                cudaMemcpyAsync(reinterpret_cast<double *>(d_coef_ + (jnd - 1)), d_scal_ + kAlpha, sizeof(double),
+                                cudaMemcpyDeviceToDevice, st_);
+                Recur<C> none;
+                int pid = pbeg();
+                launch_update<T>(d_cols_, jnd, n_pad_, r64_, none, d_coef_, r64_, d_scal_ + kR2Post, scratch_, st_);
+                pend(pid, TRLX_K_UPDATE, (double)jnd * nrow_ * sv() + 2.0 * nrow_ * cs());
+                count_launch();
+                cudaStreamSynchronize(st_);  // g must outlive the copy
+            }
+            fl_ += 2 * jnd * nrow_ + nrow_ + nrow_;
+            double f0 = fl_;
+            const int passes = info->north;
+            stat = orth(jnd, false, 0.0, kept);
+            took_steps(1, info->north == passes + 1);
+            fl_h_ += fl_ - f0;
+            tm_end();
+            if (stat) break;
+            rotate_fp64();
         }
         // Arrow -> tridiagonal for the non-locked part (the columns up to and
         // with the first step's).

@@ -685,16 +685,14 @@ __device__ void solve(const Params &P, int pid, const Grp &G, double *dyn, long 
                 for (int i = lane; i < locked + kk; i += 32) S.alpha[i] = S.lambda[i];
                 __syncwarp();
                 if (lane == 0) {
-                    {
-                        for (int i = 0; i < kk; ++i) S.beta[locked + i] = yy[(size_t)(i + 1) * jml - 1] * S.betrot[jnd - 1];
-                        if (jml > info->ned + (info->ned / 5 + 6))
-                            core::set_locking(jml, kk, &S.alpha[locked], &S.beta[locked], yy, info->anrm, &i2);
-                        else
-                            i2 = 0;
-                        S.ctl[cJnd] = jml;       // columns recombined
-                        S.ctl[cKept] = kk;
-                        S.ctl[cLocked] = i2;     // newly locked
-                    }
+                    for (int i = 0; i < kk; ++i) S.beta[locked + i] = yy[(size_t)(i + 1) * jml - 1] * S.betrot[jnd - 1];
+                    if (jml > info->ned + (info->ned / 5 + 6))
+                        core::set_locking(jml, kk, &S.alpha[locked], &S.beta[locked], yy, info->anrm, &i2);
+                    else
+                        i2 = 0;
+                    S.ctl[cJnd] = jml;       // columns recombined
+                    S.ctl[cKept] = kk;
+                    S.ctl[cLocked] = i2;     // newly locked
                 }
             } else if (!st) {
                 double *ev = S.wrk2;

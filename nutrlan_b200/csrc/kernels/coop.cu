@@ -20,13 +20,17 @@
 // is large against |x'|, so they are carried in two doubles each (compensated
 // dot products: Ogita, Rump, Oishi 2005); a step with |delta| > 16 |x'| is
 // logged as failed (the host takes it again with the sequential kernels).
-// x' is formed by each reader from z and
-// q_k, which every block writes to global memory before the barrier.  The
-// partial sums meet in two levels: the blocks of a cluster through distributed
-// shared memory, and after the grid barrier (one arrival per cluster) every
-// block adds the clusters' sums itself, all in a fixed order.
-// Vectors written by other blocks are read through L2 (ld.global.cg).  The
-// per-step log is the one the host replays to accept or discard steps.
+// x' is formed by each reader from z and q_k, which every block writes to
+// global memory before the barrier.  The partial sums meet in two levels: the
+// blocks of a cluster through distributed shared memory, and after the grid
+// barrier (one arrival per cluster) every block adds the clusters' sums itself,
+// all in a fixed order.  Vectors written by other blocks are read through L2
+// (ld.global.cg).  The per-step log is the one the host replays to accept or
+// discard steps.
+//
+// A row of the operator has as many lanes as the average row needs, a long
+// row a warp.  Every entry gathers from two vectors, so operators with many
+// entries are better off with sweeps (coop_pays in coop.h).
 //
 // Measured (one B200), per step, against a kernel of five grid-wide barriers
 // that read the basis twice: 128^2 lattice, basis 64, 27 -> 8 us; 12^3

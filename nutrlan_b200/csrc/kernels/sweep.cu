@@ -21,10 +21,13 @@
 // accurate as in the two-kernel step.
 //
 // Bound by memory; measured against the two kernels and the normalisation
-// (one B200): 256^3 FP64, 128 steps, 427 -> 280 ms a call; 1024^2
-// complex128, 64.3 -> 39.1 ms; 101^3 FP32, 30.3 -> 16.9 ms; 2048^2
-// complex64, 82.4 -> 65.6 ms (12 FP64 FMAs and two conversions per 8 bytes:
-// the sweep itself runs at 3.0-3.5 TB/s there, 5.1-5.7 for FP64 storage).
+// (one B200): 256^3 FP64, 128 steps, 427 -> 249 ms a call (the sweeps at
+// 5.9-6.0 TB/s); 1024^2 complex128, 64.3 -> 38.8 ms; 101^3 FP32, 30.3 -> 17.0
+// ms; 2048^2 complex64, 82.4 -> 64.8 ms (12 FP64 FMAs and four conversions per
+// 8 bytes: the sweep itself runs at 3.7-3.9 TB/s there).
+//
+// A sweep takes at most 128 columns: in a larger basis the steps from there on
+// read the basis twice (the discrete kernels).
 //
 // For a 32-bit basis the working vectors stay FP64: q_{k-1} is read from its
 // FP64 copy, V T h is formed from the stored columns (h is then of the size

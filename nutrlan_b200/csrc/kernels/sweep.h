@@ -8,7 +8,7 @@
 
 namespace trlb {
 
-// Columns a sweep takes (16 warps of 8).
+// Columns a sweep takes (8 warps of 16).
 constexpr int kSweepCols = 128;
 
 // Device state of a run of sweeps; column indices are those of the basis.
