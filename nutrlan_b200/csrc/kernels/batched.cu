@@ -638,6 +638,7 @@ __device__ void solve(const Params &P, int pid, const Grp &G, double *dyn, long 
             }
         }
         if (stat) break;
+        G.sync();  // every warp has left the loop on nec and the flag as they are; both may change below
         // ---- restart or finish ------------------------------------------------
         // Lane 0 of warp 0 takes the decisions; the O(maxlan^3) eigenvector
         // work runs on the whole warp (dense_warp.cuh), then all apply.
